@@ -2,8 +2,8 @@
 
 ``build_native()`` compiles ``csrc/*.cu`` with nvcc into ``libflashquant_b200.so`` (the
 C-ABI library, no torch dependency) next to this file.  ``build_pybind()`` compiles the
-pybind11 module ``_C`` (torch tensors in, C ABI underneath) with the same nvcc.  Both skip
-the work when the outputs are newer than every source.
+extension modules ``_C`` (the reference's names, pybind11) and ``_host`` (the host side of the
+package's calls), torch tensors in, C ABI underneath.  Both skip the work when the outputs are newer than every source.
 
     python -m flashquant_b200.build            # build both
     python -m flashquant_b200.build --verbose  # also print ptxas resource usage
@@ -68,21 +68,28 @@ def build_native(verbose: bool = False, force: bool = False) -> str:
     return LIB
 
 
-def pybind_path() -> str:
+def pybind_path(name: str = "_C") -> str:
     suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
-    return os.path.join(HERE, "_C" + suffix)
+    return os.path.join(HERE, name + suffix)
+
+
+# extension modules on top of the C-ABI library: the reference's `_C` names, and the host side of
+# the package's own calls
+MODULES = {"_C": "pybind_module.cpp", "_host": "host_calls.cpp"}
 
 
 def build_pybind(verbose: bool = False, force: bool = False) -> str:
-    """Compile the pybind11 module ``flashquant_b200._C`` (needs torch headers)."""
-    out = pybind_path()
-    src = os.path.join(CSRC, "pybind_module.cpp")
-    if not os.path.exists(src):
-        raise RuntimeError("pybind_module.cpp is missing")
+    """Compile the extension modules ``_C`` and ``_host`` (need torch headers); path of ``_C``."""
     build_native(verbose=verbose, force=force)
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= max(
-            _newest_input(), os.path.getmtime(LIB)):
-        return out
+    stale = [n for n in MODULES if force or not os.path.exists(pybind_path(n)) or
+             os.path.getmtime(pybind_path(n)) < max(_newest_input(), os.path.getmtime(LIB))]
+    if stale:
+        with ThreadPoolExecutor(max_workers=len(stale)) as ex:
+            list(ex.map(lambda n: _build_module(n, verbose), stale))
+    return pybind_path()
+
+
+def _build_module(name: str, verbose: bool) -> None:
     import torch
     from torch.utils import cpp_extension as ce
 
@@ -92,20 +99,18 @@ def build_pybind(verbose: bool = False, force: bool = False) -> str:
     inc += ["-I", sysconfig.get_paths()["include"], "-I", "/usr/local/cuda/include"]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_C",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={name}",
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-           "-I", INCLUDE, *inc, src, "-o", out,
+           "-I", INCLUDE, *inc, os.path.join(CSRC, MODULES[name]), "-o", pybind_path(name),
            "-L", HERE, "-l:libflashquant_b200.so", "-Wl,-rpath,$ORIGIN",
            "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-ltorch_cuda",
            "-lc10_cuda", "-L", "/usr/local/cuda/lib64", "-lcudart",
            f"-Wl,-rpath,{torch_lib}"]
     _run(cmd, verbose)
-    return out
 
 
 if __name__ == "__main__":
     v = "--verbose" in sys.argv
     f = "--force" in sys.argv
     print(build_native(verbose=v, force=f))
-    if os.path.exists(os.path.join(CSRC, "pybind_module.cpp")):
-        print(build_pybind(verbose=v, force=f))
+    print(build_pybind(verbose=v, force=f))

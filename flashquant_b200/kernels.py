@@ -18,6 +18,20 @@ import torch
 
 from . import _native as N
 
+_host_module = None
+
+
+def _host():
+    """The extension module that makes a call whose arguments need no conversion (it returns None
+    for the others, an int for a native status, else the result)."""
+    global _host_module
+    if _host_module is None:
+        N.load()  # the message about a library that has not been built
+        from . import _host as m
+        _host_module = m
+    return _host_module
+
+
 _PART_PAD = 4  # a partial row holds head_dim + 4 floats (acc, m, l, 2 pads)
 
 
@@ -46,6 +60,12 @@ def tq4_compress(
 
     Same contract as the reference's ``tq4_compress`` (src/flashquant/kernels/compress.py:51-95).
     """
+    if out is None and rotation_T_even is not None and rotation_T_odd is not None:
+        r = _host().compress(x, rotation_T_even, rotation_T_odd, boundaries)
+        if type(r) is tuple:
+            return r
+        if r is not None:
+            N.check(r)
     N.require_cuda(x)
     n, h, d = x.shape
     dev = x.device
@@ -179,6 +199,10 @@ def cache_update(key, value, tables_k, tables_v, k_packed, k_norms, v_packed, v_
 
     ``tables_*``: (Pi^T even columns, Pi^T odd columns, boundaries, centroids, Pi) on the device.
     """
+    r = _host().cache_update(key, value, tables_k, tables_v, k_packed, k_norms, v_packed, v_norms,
+                             position, k_out, v_out, out_position, workspace)
+    if r is not None:
+        return N.check(r)
     N.require_cuda(key, value, k_packed, k_norms, v_packed, v_norms, k_out, v_out)
     b, h, s, d = key.shape
     if value.shape != key.shape or value.dtype != key.dtype:
@@ -317,6 +341,10 @@ def tq4_compress_append(key, value, kv_cache, slot_mapping, rotation, boundaries
     compress calls, eight slice copies and an index_put (src/flashquant/vllm/impl.py:220-263).
     Negative slots are skipped.
     """
+    r = _host().compress_append(key, value, kv_cache, slot_mapping, rotation, boundaries_k,
+                                boundaries_v)
+    if r is not None:
+        return N.check(r)
     key, value, stride, n, h, d, num_slots, slots = _append_common(key, value, kv_cache,
                                                                    slot_mapping)
     dev = key.device
@@ -337,6 +365,10 @@ def tq4_compress_append_qjl(key, value, kv_cache, kq_cache, slot_mapping, rotati
     Sign bits and residual norm of every K vector go to the side plane ``kq_cache``
     ``(num_blocks, block_size, H*(D/8+4))`` = [sign bits | gamma], heads in order.
     """
+    r = _host().compress_append_qjl(key, value, kv_cache, kq_cache, slot_mapping, rotation,
+                                    boundaries_k, centroids_k, boundaries_v, qjl_matrix)
+    if r is not None:
+        return N.check(r)
     key, value, stride, n, h, d, num_slots, slots = _append_common(key, value, kv_cache,
                                                                    slot_mapping)
     dev = key.device
@@ -362,7 +394,13 @@ def tq4_compress_append_qjl(key, value, kv_cache, kq_cache, slot_mapping, rotati
 # split-K paged decode
 # --------------------------------------------------------------------------------------
 
-_workspaces = {}
+# uses of the cached workspaces (one per device, stream and use)
+_DECODE, _ATTENTION, _PREFILL = 0, 1, 2
+
+
+def _workspace(device, use: int, need: int) -> torch.Tensor:
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _host().workspace(index, use, need)
 
 
 def decode_workspace(device, num_seqs: int, num_q_heads: int, num_kv_heads: int, head_dim: int,
@@ -373,12 +411,7 @@ def decode_workspace(device, num_seqs: int, num_q_heads: int, num_kv_heads: int,
                                                               head_dim, num_splits))
     # one workspace per (device, stream): calls on different streams may overlap on the GPU
     # and must not share counters or partial rows
-    key = (device.type, device.index, torch.cuda.current_stream(device).cuda_stream)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    return _workspace(device, _DECODE, need)
 
 
 def set_single_launch(enabled: bool) -> None:
@@ -440,6 +473,12 @@ def split_k_paged_decode(
     (src/flashquant/kernels/paged_decode.py:56-128): un-rotated ``q`` in, output in the
     original space, ``num_splits = 0`` picks the partition count.
     """
+    if workspace is None:
+        r = _host().paged_decode(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v,
+                                 rotation, num_kv_heads, head_dim, block_size, sm_scale, out,
+                                 num_splits)
+        if r is not None:
+            return r if type(r) is not int else N.check(r)
     dev, num_seqs, hq, d, q, block_table, seq_lens, ck, cv, rot = _decode_args(
         q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation, num_kv_heads,
         head_dim, block_size)
@@ -475,6 +514,11 @@ def split_k_paged_decode_multi(q, kv_cache, block_table, seq_lens, centroids_k, 
     (``fq_split_k_paged_decode_multi``: a small kernel writes those rows, then the decode
     launch), so nothing is de-quantised to memory.
     """
+    r = _host().paged_decode_multi(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v,
+                                   rotation, num_kv_heads, head_dim, block_size, sm_scale,
+                                   num_splits)
+    if r is not None:
+        return r if type(r) is not int else N.check(r)
     N.require_cuda(q, kv_cache, block_table, seq_lens)
     if q.dim() != 4:
         raise ValueError("q must be (num_seqs, n_q, H_q, D)")
@@ -511,6 +555,12 @@ def split_k_paged_decode_qjl(q, kv_cache, kq_cache, block_table, seq_lens, centr
     (``TurboQuantProd.estimate_inner_product``, src/flashquant/core/quantizer.py:349-370):
     ``<q,k> ~ <q,k_mse> + gamma*sqrt(pi/2)/m*<S q, signs>`` with signs and gamma read from the
     side plane ``kq_cache`` that ``tq4_compress_append_qjl`` fills."""
+    if workspace is None:
+        r = _host().paged_decode_qjl(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v,
+                                     rotation, num_kv_heads, head_dim, block_size, sm_scale, out,
+                                     num_splits, kq_cache, qjl_matrix)
+        if r is not None:
+            return r if type(r) is not int else N.check(r)
     dev, num_seqs, hq, d, q, block_table, seq_lens, ck, cv, rot = _decode_args(
         q, kv_cache, block_table, seq_lens, centroids_k, centroids_v, rotation, num_kv_heads,
         head_dim, block_size)
@@ -549,6 +599,12 @@ def paged_tq4_prefill(q, kv_cache, block_table, seq_lens, cu_seqlens_q, max_q_le
     computes after de-quantising the whole cache (src/flashquant/vllm/impl.py:265-336,
     477-509); ``workspace`` word 0 is the device status word.
     """
+    if workspace is None:
+        r = _host().paged_prefill(q, kv_cache, block_table, seq_lens, centroids_k, centroids_v,
+                                  rotation, num_kv_heads, head_dim, block_size, sm_scale, out,
+                                  cu_seqlens_q, max_q_len)
+        if r is not None:
+            return r if type(r) is not int else N.check(r)
     N.require_cuda(q, kv_cache, block_table, seq_lens, cu_seqlens_q)
     dev = q.device
     total, hq, d = q.shape
@@ -568,7 +624,7 @@ def paged_tq4_prefill(q, kv_cache, block_table, seq_lens, cu_seqlens_q, max_q_le
     lib = N.load()
     need = lib.fq_paged_tq4_prefill_workspace_bytes(total, hq, d)
     if workspace is None:
-        workspace = torch.zeros(max(need, 256), dtype=torch.uint8, device=dev)
+        workspace = _workspace(dev, _PREFILL, need)
     N.check(lib.fq_paged_tq4_prefill(
         N.ptr(q), N.dtype_code(q.dtype), N.ptr(kv_cache), N.ptr(block_table),
         block_table.stride(0), N.ptr(seq_lens), N.ptr(cu), N.ptr(ck), ck.numel(), N.ptr(cv),
@@ -744,9 +800,6 @@ def split_k_merge(partials: torch.Tensor, rotation: torch.Tensor, dtype: torch.d
 # fused TQ4 attention (prefill)
 # --------------------------------------------------------------------------------------
 
-_attn_workspaces = {}
-
-
 def fused_tq_attention(
     q: torch.Tensor,
     k_packed: torch.Tensor,
@@ -765,6 +818,10 @@ def fused_tq_attention(
     (src/flashquant/kernels/attention.py:53-107): ``q (B, H_Q, N_Q, D)``, packed codes
     ``(B, H_KV, N_KV, D/2)``, norms ``(B, H_KV, N_KV, 1)``.
     """
+    r = _host().attention(q, k_packed, k_norms, v_packed, v_norms, centroids_k, centroids_v,
+                          rotation, rotation, sm_scale, bool(is_causal))
+    if r is not None:
+        return r if type(r) is not int else N.check(r)
     N.require_cuda(q, k_packed, k_norms, v_packed, v_norms)
     b, hq, nq, d = q.shape
     _, hkv, nkv, half = k_packed.shape
@@ -781,11 +838,7 @@ def fused_tq_attention(
     out = torch.empty_like(q)
     lib = N.load()
     need = lib.fq_fused_tq_attention_workspace_bytes(b, hq, nq, d)
-    key = (dev.type, dev.index)
-    ws = _attn_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(need, dtype=torch.uint8, device=dev)
-        _attn_workspaces[key] = ws
+    ws = _workspace(dev, _ATTENTION, need)
     N.check(lib.fq_fused_tq_attention(
         N.ptr(q), N.dtype_code(q.dtype), N.ptr(kp), N.ptr(kn), N.ptr(vp), N.ptr(vn), N.ptr(ck),
         ck.numel(), N.ptr(cv), cv.numel(), N.ptr(rot), b, hq, hkv, nq, nkv, d, float(sm_scale),
@@ -828,6 +881,10 @@ def fused_tq_attention_kv(
     (src/flashquant/cache/hf_cache.py:387-414): ``[:, :, :n_kv]`` views of buffers with room
     for more tokens; keys and values carry their own rotation (seeds 42 / 43).
     """
+    r = _host().attention(q, k_packed, k_norms, v_packed, v_norms, centroids_k, centroids_v,
+                          rotation_k, rotation_v, sm_scale, bool(is_causal))
+    if r is not None:
+        return r if type(r) is not int else N.check(r)
     N.require_cuda(q, k_packed, k_norms, v_packed, v_norms)
     b, hq, nq, d = q.shape
     _, hkv, nkv, half = k_packed.shape
@@ -847,11 +904,7 @@ def fused_tq_attention_kv(
     out = torch.empty_like(q)
     lib = N.load()
     need = lib.fq_fused_tq_attention_workspace_bytes(b, hq, nq, d)
-    key = (dev.type, dev.index)
-    ws = _attn_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(need, dtype=torch.uint8, device=dev)
-        _attn_workspaces[key] = ws
+    ws = _workspace(dev, _ATTENTION, need)
     N.check(lib.fq_fused_tq_attention_kv(
         N.ptr(q), N.dtype_code(q.dtype), N.ptr(k_packed), N.ptr(k_norms), N.ptr(v_packed),
         N.ptr(v_norms), N.ptr(ck), ck.numel(), N.ptr(cv), cv.numel(), N.ptr(rk), N.ptr(rv), b, hq,
@@ -861,6 +914,5 @@ def fused_tq_attention_kv(
 
 
 def attention_workspace_status(device) -> int:
-    """Device status word of the cached attention workspace (0 = no error)."""
-    ws = _attn_workspaces.get((device.type, device.index))
-    return 0 if ws is None else workspace_status(ws)
+    """Device status word of the current stream's attention workspace (0 = no error)."""
+    return workspace_status(_workspace(device, _ATTENTION, 0))

@@ -1,0 +1,58 @@
+"""The direct call path (arguments the kernels take as they are) and the converting one (constants
+on the CPU, other layouts) give the same bits, and wrong arguments still raise."""
+
+import pytest
+import torch
+
+import flashquant_b200 as fq
+from flashquant_b200 import kernels as K
+from flashquant_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_direct_and_converting_calls_agree(consts, dtype):
+    w = W.decode_workload(seq_lens=[1, 40, 700], num_q_heads=32, num_kv_heads=8, cfg=61, dtype=dtype)
+    k, v = (t.to(DEV) for t in W.make_kv(w.total_tokens, 8, 128, 61, dtype))
+    slots, bt, sl, q = (t.to(DEV) for t in (w.slot_mapping, w.block_table, w.seq_lens, w.q))
+    host = [consts[n].contiguous() for n in ("rotation_128_0", "boundaries_128_3",
+                                             "centroids_128_3", "boundaries_128_4",
+                                             "centroids_128_4", "qjl_128_0")]
+    got = []
+    for c in (host, [t.to(DEV) for t in host]):
+        rot, bk, ck, bv, cv, qjl = c
+        cache = torch.zeros(w.num_blocks, 16, 8 * 136, dtype=torch.uint8, device=DEV)
+        plane = torch.zeros(w.num_blocks, 16, 8 * 20, dtype=torch.uint8, device=DEV)
+        fq.tq4_compress_append(k, v, cache, slots, rot, bk, bv)
+        one = cache.clone()
+        fq.tq4_compress_append_qjl(k, v, cache, plane, slots.int(), rot, bk, ck, bv, qjl)
+        geo = (8, 128, 16)
+        out = fq.split_k_paged_decode(q, cache, bt, sl, ck, cv, rot, *geo)
+        multi = fq.split_k_paged_decode_multi(q[:, None].contiguous(), cache, bt, sl, ck, cv, rot,
+                                              *geo)
+        cu = torch.tensor([0, 1, 2, 3], dtype=torch.int32, device=DEV)
+        pre = fq.paged_tq4_prefill(q, cache, bt, sl, cu, 1, ck, cv, rot, *geo)
+        got.append((one, cache, plane, out, multi, pre))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+def test_strided_tokens_and_streams(consts):
+    """Keys and values as slices of one projection, and a second stream with its own workspace."""
+    rot, bk, bv = (consts[n].contiguous().to(DEV) for n in
+                   ("rotation_128_0", "boundaries_128_3", "boundaries_128_4"))
+    qkv = torch.randn(33, 3 * 8, 128, device=DEV).to(torch.bfloat16)
+    k, v = qkv[:, 8:16], qkv[:, 16:]
+    slots = torch.arange(33, device=DEV)
+    a, b = (torch.zeros(3, 16, 8 * 136, dtype=torch.uint8, device=DEV) for _ in range(2))
+    fq.tq4_compress_append(k, v, a, slots, rot, bk, bv)
+    fq.tq4_compress_append(k.contiguous(), v.contiguous(), b, slots, rot, bk, bv)
+    assert torch.equal(a, b)
+    first = K.decode_workspace(torch.device(DEV), 1, 8, 8, 128, 0)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        assert K.decode_workspace(torch.device(DEV), 1, 8, 8, 128, 0).data_ptr() != first.data_ptr()
+    assert K.decode_workspace(torch.device(DEV), 1, 8, 8, 128, 0).data_ptr() == first.data_ptr()
+    with pytest.raises(ValueError):
+        fq.tq4_compress_append(k, v, a[..., :-1].contiguous(), slots, rot, bk, bv)
