@@ -1,9 +1,9 @@
 // One update of a contiguous compressed cache in one host call: the new keys and values are
 // compressed into their rows of the pre-allocated buffers and, unless the caller attends over
 // the codes directly, those rows are de-quantised to the original space and written behind
-// the tokens the caller already holds.  Four launches on one stream for a few new rows (the
-// back-rotation expands the codes on its way in), six otherwise; no allocation, no
-// synchronisation.
+// the tokens the caller already holds.  Launches on one stream: one for a few new rows and two for
+// many without the read-back; four (the back-rotation expands the codes on its way in) and
+// six with it.  No allocation, no synchronisation.
 #include "fq_common.cuh"
 
 using namespace fq;
@@ -51,7 +51,22 @@ extern "C" int fq_cache_update(
     FQ_REQUIRE(n_centroids >= 1 && n_centroids <= 16, FQ_ERR_INVALID_ARGUMENT,
                "n_centroids %d outside [1, 16]", n_centroids);
   }
-  int rc = fq_tq4_compress_into(key, dtype, rot_T_even_k, rot_T_odd_k, boundaries, n_boundaries,
+  int rc = FQ_OK;
+  if (!dequantise && rot_T_even_k && rot_T_odd_k && rot_T_even_v && rot_T_odd_v && boundaries &&
+      n_boundaries >= 1 && n_boundaries <= 15 && aligned(key, dtype == FQ_F32 ? 16 : 8) &&
+      aligned(value, dtype == FQ_F32 ? 16 : 8) && aligned(k_norms, 4) && aligned(v_norms, 4)) {
+    CompressPair u{};
+    u.src[0] = key; u.src[1] = value;
+    u.even[0] = rot_T_even_k; u.odd[0] = rot_T_odd_k;
+    u.even[1] = rot_T_even_v; u.odd[1] = rot_T_odd_v;
+    u.boundaries = boundaries; u.n_boundaries = n_boundaries;
+    u.packed[0] = k_packed; u.packed[1] = v_packed;
+    u.norms[0] = k_norms; u.norms[1] = v_norms;
+    u.n_segments = n_segments; u.n_new = n_new; u.capacity = capacity; u.position = position;
+    u.head_dim = head_dim;
+    if (compress_pair_few(u, int(dtype), static_cast<cudaStream_t>(stream), rc)) return rc;
+  }
+  rc = fq_tq4_compress_into(key, dtype, rot_T_even_k, rot_T_odd_k, boundaries, n_boundaries,
                                 k_packed, k_norms, n_segments, n_new, capacity, position,
                                 head_dim, stream);
   if (rc != FQ_OK) return rc;

@@ -55,6 +55,9 @@ struct CompressArgs {
   uint32_t seg_len;
   int64_t seg_stride;
   int64_t seg_offset;
+  // source 1 by another rotation (null: mat_a / mat_b); compress_few_kernel only
+  const float* mat_a1;
+  const float* mat_b1;
 };
 
 __device__ __forceinline__ int64_t segment_row(const CompressArgs& p, uint32_t tok) {
@@ -772,6 +775,10 @@ __global__ void __launch_bounds__(kCoopThreads, QJL ? 1 : 2) compress_coop_kerne
   }
 }
 
+}  // namespace fq
+#include "compress_few.cuh"
+namespace fq {
+
 // below this many tiles the CTA-per-tile kernel is the faster one (measured cross-over at
 // about 1000 tiles: it starts in 12 us and needs 6.6 us per wave of tiles, the warp-per-tile
 // kernel 30 us and 33 us per eight tiles and SM)
@@ -820,6 +827,9 @@ static int launch_compress_t(const CompressArgs& a, cudaStream_t stream) {
   const int64_t n_vec = a.n_tokens * a.heads;
   const int64_t tiles = (n_vec + kTileRows - 1) / kTileRows;
   if (tiles == 0) return FQ_OK;
+  if (n_vec * a.n_src <= kFewMaxVectors && aligned(a.mat_a, 16) && aligned(a.mat_b, 16) &&
+      aligned(a.qjl, 16))
+    return launch_compress_few<D, DT, QJL>(a, n_vec, stream);
   if (tiles < kCoopMaxTiles) return launch_compress_coop<D, DT, QJL>(a, tiles, stream);
   FQ_REQUIRE(n_vec < (int64_t(1) << 31) - 16 * 4096, FQ_ERR_UNSUPPORTED,
              "compress: %lld vectors in one call (at most 2^31)", (long long)n_vec);
@@ -850,6 +860,29 @@ static int launch_compress(const CompressArgs& a, int dtype, int head_dim, bool 
                : launch_compress_d<64, false>(a, dtype, stream);
   return fail(FQ_ERR_UNSUPPORTED, "head_dim %d: the compress kernels are built for 64 and 128",
               head_dim);
+}
+
+// A contiguous cache's few new vectors in one launch, keys and values with their own rotations.
+// False: too many, or not laid out for it (the caller goes tensor by tensor).
+bool compress_pair_few(const CompressPair& u, int dtype, cudaStream_t stream, int& rc) {
+  const int64_t n_vec = u.n_segments * u.n_new;
+  if (2 * n_vec > kFewMaxVectors || (u.head_dim != 64 && u.head_dim != 128)) return false;
+  CompressArgs a{};
+  a.n_src = 2;
+  a.n_tokens = n_vec; a.heads = 1; a.token_stride = u.head_dim;
+  a.mat_a = u.even[0]; a.mat_b = u.odd[0]; a.mat_a1 = u.even[1]; a.mat_b1 = u.odd[1];
+  a.rot_split = 1;
+  for (int s = 0; s < 2; ++s) {
+    a.src[s] = u.src[s];
+    a.bnd[s] = u.boundaries; a.nb[s] = u.n_boundaries;
+    a.code[s] = u.packed[s];
+    a.norm[s] = reinterpret_cast<uint8_t*>(u.norms[s]);
+    if (!aligned(u.even[s], 16) || !aligned(u.odd[s], 16) || !aligned(u.packed[s], 4)) return false;
+  }
+  a.code_row_stride = u.head_dim / 2; a.norm_row_stride = 4;
+  a.seg_len = uint32_t(u.n_new); a.seg_stride = u.capacity; a.seg_offset = u.position;
+  rc = launch_compress(a, dtype, u.head_dim, false, stream);
+  return true;
 }
 
 static int elem_bytes(int dtype) { return dtype == FQ_F32 ? 4 : 2; }

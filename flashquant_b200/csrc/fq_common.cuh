@@ -374,6 +374,19 @@ int rotate_back_from_codes(const uint8_t* codes, const float* norms, const float
                            int n_centroids, RowMap in_map, int dtype, const float* rotation,
                            void* out, int64_t n_rows, int head_dim, cudaStream_t stream,
                            RowMap out_map);
+// compress.cu: keys [0] and values [1] of a contiguous cache's few new vectors in one launch
+struct CompressPair {
+  const void* src[2];
+  const float *even[2], *odd[2];  // Pi^T, even and odd columns
+  const float* boundaries;
+  int n_boundaries;
+  uint8_t* packed[2];
+  float* norms[2];
+  int64_t n_segments, n_new, capacity, position;
+  int head_dim;
+};
+bool compress_pair_few(const CompressPair& u, int dtype, cudaStream_t stream, int& rc);
+
 // decompress.cu: codes (rows through in_map) -> rotated-space values, contiguous
 int decompress_rows(const uint8_t* packed, const float* norms, const float* centroids,
                     int n_centroids, void* out, int out_dtype, int64_t n_vectors, int head_dim,
