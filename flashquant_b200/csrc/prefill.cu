@@ -1,8 +1,12 @@
-// Fused causal TQ4 FlashAttention-2 prefill for sm_100a on the 5th-generation tensor cores.
+// Fused TQ4 FlashAttention-2 for sm_100a on the 5th-generation tensor cores.
 //
-// One CTA of 256 threads owns 128 query rows of one (batch, query head) - two threads per
-// row, each with half of the columns - and walks the KV sequence in tiles of 64 tokens,
-// skipping tiles above the causal diagonal.  Per tile:
+// Two kernels: prefill_pair_kernel (prefill_pair.cuh) for calls with many query rows, contiguous
+// or paged, and prefill_attention_kernel below for one query token per sequence over a contiguous
+// cache, whose keys are cut into slices so that the CTAs fill the GPU.
+//
+// prefill_attention_kernel: one CTA of 256 threads owns the query rows of one (batch, KV head) - two
+// threads per row, each with half of the columns - and walks its slice in tiles of 64 tokens.
+// Per tile:
 //   * the packed K and V codes and their norms arrive by 1-D bulk copies, one tile ahead;
 //   * all threads turn codes into fp16 centroids (256-entry table of fp16 pairs) and store
 //     them as tcgen05 shared-memory operands; the norms are NOT applied here: |k| scales the
@@ -10,9 +14,8 @@
 //   * one thread issues S = Q K^T (tcgen05.mma, fp16 x fp16 -> fp32 in TMEM) - for the NEXT
 //     tile, into the other of two score buffers, so that it runs under this tile's softmax;
 //   * the two threads of row r read their halves of row r of S from TMEM (tcgen05.ld), apply
-//     |k|, the scale and - on tiles that touch the diagonal or the end - the causal mask,
-//     update the online softmax and write the fp16 weights as the A operand of the second
-//     product;
+//     |k| and the scale, update the online softmax and write the fp16 weights as the A operand
+//     of the second product;
 //   * one thread issues O += P V into TMEM, where the accumulator stays across all tiles: the
 //     reference exponent of the online softmax is raised lazily (only when a row's scores
 //     outgrow it by more than 6 bits), and only then do the threads of that warp rescale their
@@ -206,24 +209,7 @@ struct PrefillSmem {
 //                 issue O += P V(t)                                             (tensor)
 // so a score product always has a whole softmax to complete in, and the PV product the next
 // tile's key dequantisation.  Codes and norms arrive by bulk copies one tile ahead.
-// 16 or 4 bytes global -> shared without a register in between; `valid` false writes zeros
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
-               "r"(valid ? 16u : 0u)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src),
-               "r"(valid ? 4u : 0u)
-               : "memory");
-}
-// the barrier receives one arrival from this thread once all its copies above have landed
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-template <int D, bool PAGED>
+template <int D>
 __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(PrefillArgs p) {
   using S = PrefillSmem<D>;
   constexpr uint32_t kIdescS = umma_idesc(kPfM, kPfN, false);
@@ -255,30 +241,9 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   const int group = p.hq / p.hkv;
   const int hkv = hq / group;
   const int m0 = m_tile * kPfM;
-  // paged mode: this sequence's query tokens and keys; ctx keys precede the first query token
-  int q_first = 0, q_len = p.nq, kv_len = p.nkv, ctx = 0;
-  bool clamped = false;
-  if constexpr (PAGED) {
-    q_first = p.cu_q[b];
-    q_len = p.cu_q[b + 1] - q_first;
-    kv_len = p.seq_lens[b];
-    const int64_t room = p.bt_stride * int64_t(p.block_size);  // keys a block-table row can name
-    if (kv_len > room) {
-      kv_len = int(room);
-      clamped = true;
-    }
-    ctx = kv_len - q_len;
-    // a chunk outside the query tokens is not touched; one longer than the grid covers is cut
-    const bool outside = q_first < 0 || q_len < 0 || int64_t(q_first) + q_len > p.total_q;
-    if ((outside || q_len > int(gridDim.x) * kPfM) && m_tile == 0 && tid == 0 && p.status)
-      atomicOr(p.status, FQ_DEV_BAD_LENGTH);
-    if (outside || m0 >= q_len) return;  // the grid is sized for the longest chunk
-  }
-  const int rows = q_len - m0 < kPfM ? q_len - m0 : kPfM;
+  const int rows = p.nq - m0 < kPfM ? p.nq - m0 : kPfM;
 
-  int kv_end = kv_len;
-  if (p.causal && ctx + m0 + rows < kv_end) kv_end = ctx + m0 + rows;
-  if (kv_end < 0) kv_end = 0;
+  int kv_end = p.nkv;
   // a slice of the keys: move the bases, the loop below then sees tokens 0 .. kv_end of it
   const int kv_begin = split * p.split_tokens;
   if (split_mode) {
@@ -287,20 +252,19 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   }
   const int n_tiles = (kv_end + kPfN - 1) / kPfN;
 
-  const int64_t kv_row0 = PAGED ? 0 : (int64_t(b) * p.hkv + hkv) * p.kv_stride + kv_begin;
-  const uint8_t* kc_base = PAGED ? nullptr : p.k_packed + kv_row0 * (D / 2);
-  const uint8_t* vc_base = PAGED ? nullptr : p.v_packed + kv_row0 * (D / 2);
-  const float* kn_base = PAGED ? nullptr : p.k_norms + kv_row0;
-  const float* vn_base = PAGED ? nullptr : p.v_norms + kv_row0;
-  // norms ride along with the codes when a bulk copy can take them (16-byte granularity);
-  // in paged mode they always arrive with the codes
+  const int64_t kv_row0 = (int64_t(b) * p.hkv + hkv) * p.kv_stride + kv_begin;
+  const uint8_t* kc_base = p.k_packed + kv_row0 * (D / 2);
+  const uint8_t* vc_base = p.v_packed + kv_row0 * (D / 2);
+  const float* kn_base = p.k_norms + kv_row0;
+  const float* vn_base = p.v_norms + kv_row0;
+  // norms ride along with the codes when a bulk copy can take them (16-byte granularity)
   const bool norm_bulk =
-      PAGED || ((reinterpret_cast<uintptr_t>(kn_base) | reinterpret_cast<uintptr_t>(vn_base)) & 15) == 0;
+      ((reinterpret_cast<uintptr_t>(kn_base) | reinterpret_cast<uintptr_t>(vn_base)) & 15) == 0;
 
   // ---- set-up ---------------------------------------------------------------------------
   if (tid == 0) {
-    mbar_init(bar_k, PAGED ? kPfThreads : 1);  // paged: one arrival per thread and tile
-    mbar_init(bar_v, PAGED ? kPfThreads : 1);
+    mbar_init(bar_k, 1);
+    mbar_init(bar_v, 1);
     mbar_init(bar_s, 1);
     mbar_init(bar_s + 1, 1);
     mbar_init(bar_o, 1);
@@ -320,13 +284,11 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   }
   // Q tile -> [k-chunk][row][16 B]
   {
-    const __half* qsrc = PAGED ? p.q_rot + (int64_t(q_first + m0) * p.hq + hq) * D
-                               : p.q_rot + ((int64_t(b) * p.hq + hq) * p.nq + m0) * D;
-    const int64_t q_pitch = PAGED ? int64_t(p.hq) * D : D;
+    const __half* qsrc = p.q_rot + ((int64_t(b) * p.hq + hq) * p.nq + m0) * D;
     for (int i = tid; i < kPfM * int(S::kChunks); i += kPfThreads) {
       const int r = i / int(S::kChunks), kc = i % int(S::kChunks);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (r < rows) v = *reinterpret_cast<const uint4*>(qsrc + int64_t(r) * q_pitch + kc * 8);
+      if (r < rows) v = *reinterpret_cast<const uint4*>(qsrc + int64_t(r) * D + kc * 8);
       *reinterpret_cast<uint4*>(smem + S::kOffQ + kc * S::kSlabQ + r * 16) = v;
     }
   }
@@ -365,45 +327,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     if (with_norms)
       bulk_g2s(is_k ? nk_raw : nv_raw, (is_k ? kn_base : vn_base) + t0, kPfN * 4, bar);
   };
-  // Paged mode, ALL threads: the tile's codes and norms gathered through the block table, 16
-  // bytes per thread (thread = (token, quarter of its 64 code bytes)) and one norm for the
-  // first 64 threads; tokens past the end arrive as zeros.  The token rows of a tile (byte
-  // offsets into the cache, -1 past the end) are looked up one tile before its key gather, so
-  // that no gather waits for a block-table load; the value gather of the same tile, one
-  // iteration later, reuses them.
-  [[maybe_unused]] bool bad_page = false;
-  [[maybe_unused]] auto token_row = [&](int t) -> int64_t {
-    if (t >= kv_end) return -1;
-    const int page = t / p.block_size;
-    int64_t phys = p.block_table[int64_t(b) * p.bt_stride + page];
-    if (phys < 0 || phys >= p.num_blocks) {  // reported, not followed
-      phys = 0;
-      bad_page = true;
-    }
-    return (phys * p.block_size + (t - page * p.block_size)) * int64_t(p.hkv * (D + 8));
-  };
-  struct TileRows {
-    int64_t code, norm;  // rows of token tid/4 (codes) and of token tid (norm; threads 0..63)
-  };
-  [[maybe_unused]] auto tile_rows = [&](int tile) {
-    TileRows r;
-    r.code = token_row(tile * kPfN + (tid >> 2));
-    r.norm = tid < kPfN ? token_row(tile * kPfN + tid) : -1;
-    return r;
-  };
-  [[maybe_unused]] auto gather_codes = [&](const TileRows& r, bool is_k) {
-    const int piece = tid & 3;
-    const int code_off = (is_k ? 0 : p.hkv * (D / 2 + 4)) + hkv * (D / 2);
-    const int norm_off = (is_k ? 0 : p.hkv * (D / 2 + 4)) + p.hkv * (D / 2) + 4 * hkv;
-    cp_async16(smem_u32(smem + S::kOffRaw + (is_k ? 0 : S::kRawTile)) + tid * 16,
-               p.kv_cache + (r.code < 0 ? 0 : r.code) + code_off + piece * 16, r.code >= 0);
-    if (tid < kPfN)
-      cp_async4(smem_u32(is_k ? nk_raw : nv_raw) + tid * 4,
-                p.kv_cache + (r.norm < 0 ? 0 : r.norm) + norm_off, r.norm >= 0);
-    cp_async_arrive(is_k ? bar_k : bar_v);
-  };
-  // rows of the tile whose values are gathered next / whose keys are gathered next
-  [[maybe_unused]] TileRows rows_v{-1, -1}, rows_k{-1, -1};
   // all threads: codes of the landed tile -> fp16 operand tile at `op_off`
   auto dequantise = [&](int tile, bool is_k, uint32_t op_off) {
     const int n_tok = tile_tokens(tile);
@@ -441,7 +364,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   // threads 0..63: the norm of token `tid` of the tile, from the bulk copy or from memory
   auto tile_norm = [&](int tile, bool is_k) {
     const int t0 = tile * kPfN, n_tok = tile_tokens(tile);
-    if (PAGED || (norm_bulk && n_tok == kPfN)) return (is_k ? nk_raw : nv_raw)[tid];
+    if (norm_bulk && n_tok == kPfN) return (is_k ? nk_raw : nv_raw)[tid];
     return tid < n_tok ? (is_k ? kn_base : vn_base)[t0 + tid] : 0.f;
   };
   auto issue_scores = [&](int tile) {  // thread 0
@@ -461,13 +384,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
 
   // ---- prologue: K(0) -> operand, S(0) issued, K(1) and V(0) on their way ------------------
   if (n_tiles > 0) {
-    if constexpr (PAGED) {
-      rows_v = tile_rows(0);
-      gather_codes(rows_v, true);
-      gather_codes(rows_v, false);
-      rows_v = tile_rows(1);  // keys of tile 1 below, its values in iteration 0
-      rows_k = tile_rows(2);
-    } else if (tid == 0) {
+    if (tid == 0) {
       issue_codes(0, true);
       issue_codes(0, false);
     }
@@ -482,9 +399,8 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     if (tid == 0 && !dead) {
       tc_fence_after();
       issue_scores(0);
-      if (!PAGED && n_tiles > 1) issue_codes(1, true);
+      if (n_tiles > 1) issue_codes(1, true);
     }
-    if (PAGED && n_tiles > 1) gather_codes(rows_v, true);
   }
 
   for (int tile = 0; tile < n_tiles && !dead; ++tile) {
@@ -517,16 +433,8 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     if (tid == 0 && !dead) {
       tc_fence_after();
       if (more) issue_scores(tile + 1);  // runs while this tile's softmax does
-      if constexpr (!PAGED) {
-        if (tile + 2 < n_tiles) issue_codes(tile + 2, true);
-        if (more) issue_codes(tile + 1, false);
-      }
-    }
-    if constexpr (PAGED) {
-      if (tile + 2 < n_tiles) gather_codes(rows_k, true);
-      if (more) gather_codes(rows_v, false);
-      rows_v = rows_k;                // tile + 2: its values go in the next iteration
-      rows_k = tile_rows(tile + 3);   // looked up now, used in the next iteration
+      if (tile + 2 < n_tiles) issue_codes(tile + 2, true);
+      if (more) issue_codes(tile + 1, false);
     }
     // ---- S(t), issued one iteration ago -----------------------------------------------------
     if (!mbar_wait(bar_s + (tile & 1), (tile >> 1) & 1)) dead = true;
@@ -537,7 +445,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     // ---- online softmax on row `row` ---------------------------------------------------------
     // A tile that lies wholly below the diagonal of every row of the CTA and is full needs no
     // masking: the common case gets a loop body without predicates.
-    const bool unmasked = n_tok == kPfN && (!p.causal || t0 + kPfN - 1 <= m0 + ctx);
+    const bool unmasked = n_tok == kPfN;
     // pass 1: row maximum of logit*log2e + clamped log2|v| over this thread's half of the tile
     float mx = -INFINITY;
     auto row_max = [&](auto masked) {
@@ -554,7 +462,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
           float e = fmaf(sv[j + u], nk[u], lv[u]);
           if constexpr (decltype(masked)::value) {
             const int col = c0 + j + u;
-            const bool ok = col < n_tok && (!p.causal || t0 + col <= q_pos + ctx);
+            const bool ok = col < n_tok;
             e = ok ? e : -INFINITY;
           }
           mx = fmaxf(mx, e);
@@ -608,7 +516,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
           float pe = fast_exp2(fmaf(sv[j + u], nk[u], neg_m));
           if constexpr (decltype(masked)::value) {
             const int col = c0 + j + u;
-            const bool ok = col < n_tok && (!p.causal || t0 + col <= q_pos + ctx);
+            const bool ok = col < n_tok;
             pe = ok ? pe : 0.f;
           }
           l_run += pe;
@@ -645,16 +553,12 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
 
   // ---- epilogue: normalise, round, store the rotated-space row -----------------------------
   if (dead && tid == 0 && p.status) atomicOr(p.status, FQ_DEV_WAIT_TIMEOUT);
-  if constexpr (PAGED) {
-    if ((bad_page || clamped) && p.status) atomicOr(p.status, FQ_DEV_BAD_BLOCK_INDEX);
-  }
   {
     __syncthreads();  // the last tile's maxima have been read
     xch[tid] = l_run;
     __syncthreads();
     const float l_row = l_run + xch[tid ^ kPfM];  // both halves of the row
-    const int64_t row_global = PAGED ? int64_t(q_first + q_pos) * p.hq + hq
-                                     : (int64_t(b) * p.hq + hq) * p.nq + q_pos;
+    const int64_t row_global = (int64_t(b) * p.hq + hq) * p.nq + q_pos;
     // 2^-kPfPScaleLog2, and 1/l unless the rows of the slices are still to be merged
     const float inv = split_mode ? 1.f / 256.f : (l_row > 0.f ? 1.f / (l_row * 256.f) : 0.f);
     float* dst = split_mode ? p.part + (int64_t(split) * p.total_rows + row_global) * (D + 4)
@@ -676,10 +580,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           o[j] *= inv;
-          // the reference's attention over de-quantised pages returns rows of the activation
-          // type, which it then rotates (src/flashquant/vllm/impl.py:477-509): round here too
-          if (p.round_out == FQ_BF16) o[j] = __bfloat162float(__float2bfloat16_rn(o[j]));
-          if (p.round_out == FQ_F16) o[j] = __half2float(__float2half_rn(o[j]));
         }
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
@@ -690,6 +590,10 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, kPfTmemCols);
 }
+
+}  // namespace fq
+#include "prefill_pair.cuh"
+namespace fq {
 
 __global__ void __launch_bounds__(kScaleThreads) centroid_scale_kernel(
     const float* __restrict__ cent_k, int nck, const float* __restrict__ cent_v, int ncv,
@@ -739,10 +643,10 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restr
 // ------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------
-template <int D, bool PAGED = false>
+template <int D>
 static int launch_prefill_t(const PrefillArgs& a, cudaStream_t stream) {
   using S = PrefillSmem<D>;
-  auto kern = prefill_attention_kernel<D, PAGED>;
+  auto kern = prefill_attention_kernel<D>;
   static thread_local int set_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -760,6 +664,30 @@ static int launch_prefill_t(const PrefillArgs& a, cudaStream_t stream) {
   prefill_merge_kernel<D><<<unsigned((a.total_rows + 7) / 8), 256, 0, stream>>>(
       a.part, a.n_splits, a.total_rows, a.o_rot);
   return check_launch("prefill merge kernel launch");
+}
+
+// Many query rows: grid (head pairs or heads, sequences, query tiles).
+template <bool PAGED>
+static int launch_prefill_pair(const PrefillArgs& a, cudaStream_t stream) {
+  auto kern = prefill_pair_kernel<PAGED>;
+  static thread_local int set_dev = -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (set_dev != dev) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(PairSmem::kBytes));
+    if (e != cudaSuccess)
+      return fail(FQ_ERR_CUDA, "prefill: shared memory opt-in of %u bytes refused: %s",
+                  PairSmem::kBytes, cudaGetErrorString(e));
+    set_dev = dev;
+  }
+  const bool two_heads = ((a.hq / a.hkv) & 1) == 0;
+  const int rows = two_heads ? 128 : 256;
+  const dim3 grid(two_heads ? a.hq / 2 : a.hq, a.batch, (a.nq + rows - 1) / rows);
+  FQ_REQUIRE(grid.y <= 65535 && grid.z <= 65535, FQ_ERR_UNSUPPORTED,
+             "prefill: %u sequences, %u query tiles (at most 65535 of each)", grid.y, grid.z);
+  kern<<<grid, kPpThreads, PairSmem::kBytes, stream>>>(a);
+  return check_launch("prefill attention kernel launch");
 }
 
 // beta_k, beta_v for the launch that follows: found in (or left at) bytes 64..255 of the
@@ -876,7 +804,8 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
   }
   rc = centroid_scales(a, ws, stream);
   if (rc != FQ_OK) return rc;
-  rc = launch_prefill_t<128>(a, stream);
+  rc = n_q == 1 && group <= kPfM ? launch_prefill_t<128>(a, stream)
+                                 : launch_prefill_pair<false>(a, stream);
   if (rc != FQ_OK) return rc;
   if (a.n_splits > 1 && a.o_rot == nullptr)
     return rotate_back_merged(a.part, a.n_splits, dtype, rotation_v, out, rows, head_dim, stream);
@@ -985,7 +914,7 @@ extern "C" int fq_paged_tq4_prefill(const void* q, fq_dtype dtype, const uint8_t
   a.total_q = total_q_tokens;
   rc = centroid_scales(a, ws, s);
   if (rc != FQ_OK) return rc;
-  rc = launch_prefill_t<128, true>(a, s);
+  rc = launch_prefill_pair<true>(a, s);
   if (rc != FQ_OK) return rc;
   return rotate_back(o_rot, dtype, rotation, out, rows, head_dim, s);
 }
