@@ -142,11 +142,4 @@ __device__ __forceinline__ void scale_centroid_tables(unsigned char* cent, int n
   scale_sync();
 }
 
-
-// The search as a kernel of its own: one CTA of kScaleThreads threads; leaves (or finds) the
-// record at `cache` (32 centroids, beta_k, beta_v, magic, table sizes).
-__global__ void __launch_bounds__(kScaleThreads) centroid_scale_kernel(
-    const float* __restrict__ cent_k, int nck, const float* __restrict__ cent_v, int ncv,
-    uint32_t* __restrict__ cache);
-
 }  // namespace fq

@@ -41,8 +41,8 @@ constexpr int kPfM = 128;       // query rows per CTA
 constexpr int kPfN = 64;        // KV tokens per tile
 constexpr int kPfThreads = 256;  // two threads per query row: each takes half of the columns
 constexpr int kPfTmemCols = 256;
-constexpr float kPfPScaleLog2 = 8.f;  // fp16 weights are scaled by 2^8 ...
-constexpr float kPfMaxSlack = 6.f;    // ... and may exceed 1 by 2^6 before the reference exponent is raised
+// fp16 weights are scaled by 2^8 and may exceed 1 by 2^6 before the reference exponent is raised
+constexpr float kPfMaxSlack = 6.f;
 
 // ---- tcgen05 wrappers -------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* holder_smem, uint32_t cols) {
@@ -163,10 +163,15 @@ struct PrefillArgs {
   int split_tokens;
   int64_t total_rows;
   float* part;
-  // Paged, variable-length mode (PAGED kernel): q_rot / o_rot are (tokens, Hq, D); sequence b
-  // owns query tokens cu_q[b] .. cu_q[b+1] - the LAST ones of its seq_lens[b] keys, so query i
-  // sees keys 0 .. seq_lens[b] - q_len + i - and its keys and values sit in the pages
-  // block_table[b][*] of the packed cache ([K codes | K norms | V codes | V norms] per token).
+  // prefill_pair_kernel only
+  const void* q_src;                // queries as given
+  void* out;
+  const unsigned char* planes_q;    // operand planes of the key rotation ...
+  const unsigned char* planes_o;    // ... and of the value rotation (attention_prep_kernel)
+  // Its paged, variable-length form: q and out are (tokens, Hq, D); sequence b owns query tokens
+  // cu_q[b] .. cu_q[b+1] - the LAST ones of its seq_lens[b] keys, so query i sees keys 0 ..
+  // seq_lens[b] - q_len + i - and its keys and values sit in the pages block_table[b][*] of the
+  // packed cache ([K codes | K norms | V codes | V norms] per token).
   const uint8_t* kv_cache;
   const int32_t* block_table;
   int64_t bt_stride;
@@ -174,9 +179,8 @@ struct PrefillArgs {
   const int32_t* cu_q;
   int block_size;
   int64_t num_blocks;
-  int total_q;    // query tokens in q_rot / o_rot (chunks must lie inside)
-  int round_out;  // FQ_BF16 / FQ_F16: rows are rounded to that type before they are stored
-  // beta_k, beta_v of the scaled fp16 centroid tables (centroid_scale_kernel, run just before)
+  int total_q;    // query tokens in q and out (chunks must lie inside)
+  // beta_k, beta_v of the scaled fp16 centroid tables (attention_prep_kernel, run just before)
   const float* scales;
 };
 
@@ -404,7 +408,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   }
 
   for (int tile = 0; tile < n_tiles && !dead; ++tile) {
-    const int t0 = tile * kPfN;
     const int n_tok = tile_tokens(tile);
     const bool more = tile + 1 < n_tiles;
     // ---- K(t+1): codes -> operand (the other K buffer), |k| * scale by tile parity -----------
@@ -595,21 +598,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
 #include "prefill_pair.cuh"
 namespace fq {
 
-__global__ void __launch_bounds__(kScaleThreads) centroid_scale_kernel(
-    const float* __restrict__ cent_k, int nck, const float* __restrict__ cent_v, int ncv,
-    uint32_t* __restrict__ cache) {
-  __shared__ __align__(16) unsigned char cent[kCentBytes];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 1) {
-    const int i = lane & 15;
-    float c = 0.f;
-    if (lane < 16) { if (i < nck) c = cent_k[i]; } else { if (i < ncv) c = cent_v[i]; }
-    stage_centroids(cent, c, nck, ncv, cache, lane);
-  }
-  __syncthreads();
-  scale_centroid_tables(cent, nck, ncv, tid, cache);
-}
-
 // Merge of the slices' partial rows: o = sum_i 2^(m_i - M) o_i / sum_i 2^(m_i - M) l_i with
 // M = max_i m_i (a slice without keys has m = -inf, l = 0).  32 threads per query row.
 template <int D>
@@ -667,9 +655,9 @@ static int launch_prefill_t(const PrefillArgs& a, cudaStream_t stream) {
 }
 
 // Many query rows: grid (head pairs or heads, sequences, query tiles).
-template <bool PAGED>
-static int launch_prefill_pair(const PrefillArgs& a, cudaStream_t stream) {
-  auto kern = prefill_pair_kernel<PAGED>;
+template <typename T, bool PAGED>
+static int launch_prefill_pair_t(const PrefillArgs& a, cudaStream_t stream) {
+  auto kern = prefill_pair_kernel<T, PAGED>;
   static thread_local int set_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -690,13 +678,28 @@ static int launch_prefill_pair(const PrefillArgs& a, cudaStream_t stream) {
   return check_launch("prefill attention kernel launch");
 }
 
+template <bool PAGED>
+static int launch_prefill_pair(const PrefillArgs& a, fq_dtype dtype, cudaStream_t stream) {
+  return dtype == FQ_BF16 ? launch_prefill_pair_t<__nv_bfloat16, PAGED>(a, stream)
+                          : launch_prefill_pair_t<__half, PAGED>(a, stream);
+}
+
+constexpr size_t kPlaneBytes = 2 * kPpTile;  // hi and lo plane of one rotation
+
 // beta_k, beta_v for the launch that follows: found in (or left at) bytes 64..255 of the
-// workspace head, the record the decode kernels keep in theirs
-static int centroid_scales(PrefillArgs& a, unsigned char* ws, cudaStream_t stream) {
+// workspace head, the record the decode kernels keep in theirs.  With rotations: their operand
+// planes behind the head, one set if both are the same matrix.
+static int attention_prep(PrefillArgs& a, unsigned char* ws, const float* rot_q, const float* rot_o,
+                          cudaStream_t stream) {
   uint32_t* cache = reinterpret_cast<uint32_t*>(ws + kScaleCacheOffset);
-  centroid_scale_kernel<<<1, kScaleThreads, 0, stream>>>(a.cent_k, a.nck, a.cent_v, a.ncv, cache);
+  unsigned char* planes = ws + 256;
+  const int sets = rot_q ? (rot_q == rot_o ? 1 : 2) : 0;
+  attention_prep_kernel<<<1 + 4 * sets, kScaleThreads, 0, stream>>>(a.cent_k, a.nck, a.cent_v, a.ncv,
+                                                                   cache, rot_q, rot_o, planes);
   a.scales = reinterpret_cast<const float*>(cache + 32);
-  return check_launch("centroid scale kernel launch");
+  a.planes_q = planes;
+  a.planes_o = sets == 2 ? planes + kPlaneBytes : planes;
+  return check_launch("attention preparation kernel launch");
 }
 
 constexpr int kPfMaxSplits = 64;  // slices of the keys for a single query token
@@ -708,7 +711,7 @@ struct PrefillWorkspace {
 static PrefillWorkspace prefill_workspace(int64_t rows, int d, bool single_token) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   PrefillWorkspace w;
-  w.q_rot_off = 256;
+  w.q_rot_off = 256 + 2 * kPlaneBytes;
   w.o_rot_off = up(w.q_rot_off + size_t(rows) * d * 2);
   w.part_off = up(w.o_rot_off + size_t(rows) * d * 4);
   w.total = single_token ? up(w.part_off + size_t(kPfMaxSplits) * rows * (d + 4) * 4) : w.part_off;
@@ -764,8 +767,7 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   __half* q_rot = reinterpret_cast<__half*>(ws + w.q_rot_off);
   float* o_rot = reinterpret_cast<float*>(ws + w.o_rot_off);
-  int rc = rotate_q_to_half(q, dtype, rotation, q_rot, rows, head_dim, stream);
-  if (rc != FQ_OK) return rc;
+  int rc = FQ_OK;
   PrefillArgs a{};
   a.q_rot = q_rot;
   a.k_packed = k_packed; a.k_norms = k_norms;
@@ -779,7 +781,14 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
   a.causal = (is_causal && n_q > 1) ? 1 : 0;  // a single query token never needs the mask
   a.status = reinterpret_cast<uint32_t*>(ws);
   const int group = num_q_heads / num_kv_heads;
-  if (n_q == 1 && group <= kPfM) {
+  const bool one_token = n_q == 1 && group <= kPfM;
+  if (!one_token) {
+    a.q_src = q;
+    a.out = out;
+    rc = attention_prep(a, ws, rotation, rotation_v, stream);
+    return rc != FQ_OK ? rc : launch_prefill_pair<false>(a, dtype, stream);
+  }
+  {
     // One query token: the query heads of a KV group become the rows of one query tile
     // ((B, Hq, 1, D) read as (B, Hkv, group, D)), so the group's keys and values are
     // de-quantised once, and the keys are cut into slices so that the CTAs fill the GPU.
@@ -802,10 +811,9 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
       if (rotate_is_few_rows(rows)) a.o_rot = nullptr;
     }
   }
-  rc = centroid_scales(a, ws, stream);
-  if (rc != FQ_OK) return rc;
-  rc = n_q == 1 && group <= kPfM ? launch_prefill_t<128>(a, stream)
-                                 : launch_prefill_pair<false>(a, stream);
+  rc = rotate_q_to_half(q, dtype, rotation, q_rot, rows, head_dim, stream);
+  if (rc == FQ_OK) rc = attention_prep(a, ws, nullptr, nullptr, stream);
+  if (rc == FQ_OK) rc = launch_prefill_t<128>(a, stream);
   if (rc != FQ_OK) return rc;
   if (a.n_splits > 1 && a.o_rot == nullptr)
     return rotate_back_merged(a.part, a.n_splits, dtype, rotation_v, out, rows, head_dim, stream);
@@ -889,16 +897,12 @@ extern "C" int fq_paged_tq4_prefill(const void* q, fq_dtype dtype, const uint8_t
   FQ_REQUIRE(workspace && aligned(workspace, 256) && workspace_bytes >= w.total, FQ_ERR_WORKSPACE,
              "paged prefill: workspace of %zu bytes needed (256-byte aligned)", w.total);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  __half* q_rot = reinterpret_cast<__half*>(ws + w.q_rot_off);
-  float* o_rot = reinterpret_cast<float*>(ws + w.o_rot_off);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int rc = rotate_q_to_half(q, dtype, rotation, q_rot, rows, head_dim, s);
-  if (rc != FQ_OK) return rc;
   PrefillArgs a{};
-  a.q_rot = q_rot;
+  a.q_src = q;
+  a.out = out;
   a.cent_k = centroids_k; a.nck = n_centroids_k;
   a.cent_v = centroids_v; a.ncv = n_centroids_v;
-  a.o_rot = o_rot;
   a.batch = num_seqs; a.hq = num_q_heads; a.hkv = num_kv_heads; a.nq = max_q_len; a.nkv = 0;
   a.scale_log2 = sm_scale * 1.4426950408889634f;
   a.causal = 1;
@@ -910,11 +914,7 @@ extern "C" int fq_paged_tq4_prefill(const void* q, fq_dtype dtype, const uint8_t
   a.cu_q = cu_seqlens_q;
   a.block_size = block_size;
   a.num_blocks = num_blocks;
-  a.round_out = int(dtype);
   a.total_q = total_q_tokens;
-  rc = centroid_scales(a, ws, s);
-  if (rc != FQ_OK) return rc;
-  rc = launch_prefill_pair<true>(a, s);
-  if (rc != FQ_OK) return rc;
-  return rotate_back(o_rot, dtype, rotation, out, rows, head_dim, s);
+  const int rc = attention_prep(a, ws, rotation, rotation, s);
+  return rc != FQ_OK ? rc : launch_prefill_pair<true>(a, dtype, s);
 }
