@@ -11,7 +11,9 @@
 //   warps 8-11/12-15  turn key / value codes into fp16 operand tiles in shared memory (global ->
 //                     registers two tiles ahead -> look-up or byte permute -> store), once for both
 //                     query tiles;
-//   warp 16           issues every MMA: S_t = Q_t K^T and O_t += P_t V.
+//   warp 16 / 17      issues the MMAs of tile 0 / 1: S_t = Q_t K^T and O_t += P_t V.  (One warp for
+//                     both took them in a fixed order, and a tile whose weights were ready
+//                     waited for the other's: 2.9 ms.)
 // TMEM: S_0 S_1 (64 columns each), P_0 P_1 (32 each), Q_0 (64), O_0 O_1 (128 each).  Nothing in the
 // loop is a block-wide barrier.
 //
@@ -51,7 +53,7 @@ struct PairSmem {
   static constexpr uint32_t kNorm = kLut + 256 * 256;                // [8][nk | lv | vs][64]
   static constexpr uint32_t kRow = kNorm + kPpNorms * 3 * kPpN * 4;  // [2][128] query row scales
   static constexpr uint32_t kBar = kRow + 2 * 128 * 4;
-  static constexpr uint32_t kBytes = kBar + 256;
+  static constexpr uint32_t kBytes = kBar + 512;
 };
 static_assert(2 * kPpSlots * kPpHalf == 3 * kPpTile, "planes and query rows fit the rings");
 static_assert(PairSmem::kBytes <= 227 * 1024, "shared memory of one CTA");
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBar);
   uint64_t* k_full = bars;          // [3] key tile stored (128 arrivals)
-  uint64_t* k_empty = bars + 3;     // [3] its products are complete
+  uint64_t* k_empty = bars + 3;     // [3] its products are complete (one commit per query tile)
   uint64_t* v_full = bars + 6;      // [3]
   uint64_t* v_empty = bars + 9;     // [3]
   uint64_t* norm_full = bars + 12;  // [8] norms of a tile stored (128 arrivals)
@@ -266,9 +268,9 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
   uint64_t* p_full = bars + 24;     // [2] weights of query tile t stored (4 warps)
   uint64_t* o_done = bars + 26;     // [2] value product of query tile t complete
   uint64_t* planes = bars + 28;     // planes of Pi landed (prologue, epilogue)
-  uint64_t* rows_in = bars + 29;    // operand rows stored (8 warps: rotated Q, then split O)
-  uint64_t* turned = bars + 30;     // a rotation is complete (prologue, epilogue)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 31);
+  uint64_t* rows_in = bars + 29;    // [2] operand rows of tile t stored (4 warps: rotated Q, split O)
+  uint64_t* turned = bars + 31;     // [2] a rotation of tile t is complete (prologue, epilogue)
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 33);
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -318,9 +320,9 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
   if (tid == 0) {
     for (int i = 0; i < kPpSlots; ++i) {
       mbar_init(k_full + i, 128);
-      mbar_init(k_empty + i, 1);
+      mbar_init(k_empty + i, 2);
       mbar_init(v_full + i, 128);
-      mbar_init(v_empty + i, 1);
+      mbar_init(v_empty + i, 2);
     }
     for (int i = 0; i < kPpNorms; ++i) mbar_init(norm_full + i, 128);
     for (int i = 0; i < 2; ++i) {
@@ -328,10 +330,10 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
       mbar_init(s_free + i, 4);
       mbar_init(p_full + i, 4);
       mbar_init(o_done + i, 1);
+      mbar_init(rows_in + i, 4);
+      mbar_init(turned + i, 1);
     }
     mbar_init(planes, 1);
-    mbar_init(rows_in, 8);
-    mbar_init(turned, 1);
     mbar_fence_init();
     if (n_tiles > 0) {
       mbar_expect_tx(planes, 2 * kPpTile);
@@ -384,82 +386,71 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
   bool dead = false;
 
   if (warp >= 16) {
-    // ---- MMA issue --------------------------------------------------------------------------------
+    // ---- MMA issue, a warp per query tile ----------------------------------------------------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 16 && n_tiles > 0) {
+    const int t = warp - 16;
+    if (t < 2 && n_tiles > 0) {
       const bool leader = elect_one();
       const uint32_t base = smem_u32(smem);
+      const uint32_t q_rows = base + (t ? S::kQ : S::kA0);
+      const uint32_t my_s = tmem + 64 * t, my_p = tm_p + 32 * t, my_o = tm_o + 128 * t;
       auto wait = [&](uint64_t* bar, uint32_t phase) {
         if (!dead) dead = !mbar_wait_warp(bar, phase & 1, kDefaultWaitNs);
         tc_fence_after();
         return !dead;
       };
-      auto scores = [&](int t, int j) {
+      auto scores = [&](int j) {
         const uint32_t k = base + S::kK + (j % kPpSlots) * kPpHalf;
+        if (t == 0) {
 #pragma unroll
-        for (int s = 0; s < D / 16; ++s) {
-          const uint64_t kd = smem_desc(k + 2 * s * kPpSlabKV, kPpSlabKV, 128);
-          if (t == 0)
-            umma_ts(leader, tmem, tm_q0 + 8 * s, kd, kIdescS, s > 0);
-          else
-            umma_ss(leader, tmem + 64, smem_desc(base + S::kQ + 2 * s * kPpSlab, kPpSlab, 128), kd,
+          for (int s = 0; s < D / 16; ++s)
+            umma_ts(leader, my_s, tm_q0 + 8 * s, smem_desc(k + 2 * s * kPpSlabKV, kPpSlabKV, 128),
                     kIdescS, s > 0);
+        } else {
+#pragma unroll
+          for (int s = 0; s < D / 16; ++s)
+            umma_ss(leader, my_s, smem_desc(q_rows + 2 * s * kPpSlab, kPpSlab, 128),
+                    smem_desc(k + 2 * s * kPpSlabKV, kPpSlabKV, 128), kIdescS, s > 0);
         }
         umma_commit_if(leader, s_full + t);
+        umma_commit_if(leader, k_empty + j % kPpSlots);
       };
-      auto values = [&](int t, int j) {
+      auto values = [&](int j) {
         const uint32_t v = base + S::kV + (j % kPpSlots) * kPpHalf;
 #pragma unroll
         for (int s = 0; s < kPpN / 16; ++s)
-          umma_ts(leader, tm_o + 128 * t, tm_p + 32 * t + 8 * s,
-                  smem_desc(v + s * 256, 128, kPpSlabKV), kIdescO, j > 0 || s > 0);
+          umma_ts(leader, my_o, my_p + 8 * s, smem_desc(v + s * 256, 128, kPpSlabKV), kIdescO,
+                  j > 0 || s > 0);
         umma_commit_if(leader, o_done + t);
+        umma_commit_if(leader, v_empty + j % kPpSlots);
       };
       // q Pi^T: the query rows on both planes, into O_t.  (Here and in o Pi the small terms go first:
       // the accumulator is rounded at its full size only while the large ones are added.)
       if (wait(planes, 0)) {
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int s = 0; s < 2 * D / 16; ++s)
-            umma_ss(leader, tm_o + 128 * t,
-                    smem_desc(base + (t ? S::kQ : S::kA0) + 2 * (s & 7) * kPpSlab, kPpSlab, 128),
-                    smem_desc(base + S::kPi + (s < 8 ? kPpTile : 0) + 2 * (s & 7) * kPpSlab, kPpSlab, 128),
-                    kIdescQ, s > 0);
-        umma_commit_if(leader, turned);
+        for (int s = 0; s < 2 * D / 16; ++s)
+          umma_ss(leader, my_o, smem_desc(q_rows + 2 * (s & 7) * kPpSlab, kPpSlab, 128),
+                  smem_desc(base + S::kPi + (s < 8 ? kPpTile : 0) + 2 * (s & 7) * kPpSlab, kPpSlab, 128),
+                  kIdescQ, s > 0);
+        umma_commit_if(leader, turned + t);
       }
-      if (wait(rows_in, 0) && wait(k_full, 0)) {
-        scores(0, 0);
-        scores(1, 0);
-        umma_commit_if(leader, k_empty);
-      }
+      if (wait(rows_in + t, 0) && wait(k_full, 0)) scores(0);
 #pragma unroll 1
       for (int j = 0; j < n_tiles && !dead; ++j) {
         // the next tile's scores as soon as this tile's have been read
         const int n = j + 1;
-        if (n < n_tiles && wait(k_full + n % kPpSlots, n / kPpSlots)) {
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            if (wait(s_free + t, j)) scores(t, n);
-          if (!dead) umma_commit_if(leader, k_empty + n % kPpSlots);
-        }
-        if (!wait(v_full + j % kPpSlots, j / kPpSlots)) break;
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-          if (wait(p_full + t, j)) values(t, j);
-        if (!dead) umma_commit_if(leader, v_empty + j % kPpSlots);
+        if (n < n_tiles && wait(k_full + n % kPpSlots, n / kPpSlots) && wait(s_free + t, j)) scores(n);
+        if (wait(v_full + j % kPpSlots, j / kPpSlots) && wait(p_full + t, j)) values(j);
       }
       // o Pi: the rows' second terms on the hi plane, their first (both over S, P and Q_0) on the lo
       // and then the hi plane
-      if (wait(planes, 1) && wait(rows_in, 1)) {
+      if (wait(planes, 1) && wait(rows_in + t, 1)) {
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int s = 0; s < 3 * D / 16; ++s)
-            umma_ts(leader, tm_o + 128 * t, tmem + 128 * t + (s < 8 ? 64 : 0) + 8 * (s & 7),
-                    smem_desc(base + S::kPi + (s >> 3 == 1 ? kPpTile : 0) + (s & 7) * 256, 128, kPpSlab),
-                    kIdescO, s > 0);
-        umma_commit_if(leader, turned);
+        for (int s = 0; s < 3 * D / 16; ++s)
+          umma_ts(leader, my_o, tmem + 128 * t + (s < 8 ? 64 : 0) + 8 * (s & 7),
+                  smem_desc(base + S::kPi + (s >> 3 == 1 ? kPpTile : 0) + (s & 7) * 256, 128, kPpSlab),
+                  kIdescO, s > 0);
+        umma_commit_if(leader, turned + t);
       }
       if (dead && leader && p.status) atomicOr(p.status, FQ_DEV_WAIT_TIMEOUT);
     }
@@ -551,7 +542,9 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
     Raw cur = load(rows_of(0)), nxt = load(rows_of(1));
     Rows rows = rows_of(2);
     // the rings hold the planes and query rows of the first rotation until it is done
-    if (n_tiles > 0 && !mbar_wait_warp(turned, 0, kDefaultWaitNs)) dead = true;
+    if (n_tiles > 0 && !(mbar_wait_warp(turned, 0, kDefaultWaitNs) &&
+                         mbar_wait_warp(turned + 1, 0, kDefaultWaitNs)))
+      dead = true;
     const float norm_scale = dt < 64 ? p.scale_log2 * beta_k : 256.f * beta_v;
 #pragma unroll 1
     for (int j = 0; j < n_tiles && !dead; ++j) {
@@ -612,7 +605,7 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
     const uint32_t my_o = tm_o + 128 * t + lane_sel;
     // ---- the rotated query row: round to the query's type, then fp16 --------------------------------
     if (n_tiles > 0) {
-      if (!mbar_wait_warp(turned, 0, kDefaultWaitNs)) dead = true;
+      if (!mbar_wait_warp(turned + t, 0, kDefaultWaitNs)) dead = true;
       tc_fence_after();
       float unscale = 1.f / kPpPiScale;
       if constexpr (kBf16) unscale *= reinterpret_cast<const float*>(smem + S::kRow)[t * 128 + row];
@@ -637,7 +630,7 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
       if (t == 0) tc_wait_st(); else fence_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(rows_in);
+      if (lane == 0) mbar_arrive(rows_in + t);
     }
     float m_run = -INFINITY;
     uint64_t l2 = 0;  // (0, 0)
@@ -798,8 +791,8 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(rows_in);
-      if (!mbar_wait_warp(turned, 1, kDefaultWaitNs)) dead = true;
+      if (lane == 0) mbar_arrive(rows_in + t);
+      if (!mbar_wait_warp(turned + t, 1, kDefaultWaitNs)) dead = true;
       tc_fence_after();
     }
     if (dead && lane == 0 && p.status) atomicOr(p.status, FQ_DEV_WAIT_TIMEOUT);
