@@ -9,7 +9,9 @@
 // either side with any summation order) at a third of the multiply-add issue slots of an fp32
 // FMA contraction, which was the bound of this kernel before.
 //
-// A CTA of 8 warps keeps the matrices resident in shared memory as fp16 hi / lo' planes (the
+// Four kernels by number of vectors: a few (compress_few.cuh), up to a tile of 16 per SM
+// (compress_coop_kernel), many of head_dim 128 (compress_tile.cuh: tcgen05) and many of head_dim 64:
+// compress_kernel, a CTA of 8 warps that keeps the matrices resident in shared memory as fp16 hi / lo' planes (the
 // same bytes as fp32).  A warp owns a tile of 16 vectors end to end, K of the tile then V:
 // the rows come from global memory straight into MMA fragments, the products walk the column
 // tiles four at a time with the matrix fragments from ldmatrix, and the chain of the
@@ -17,7 +19,7 @@
 // operand fragment of the next product (codes -> centroids -> x_tilde -> residual -> signs) -
 // so the tile loop has no barrier and no shared-memory exchange.  The operation order is the
 // reference's (normalise, then rotate); the tie rule is bucketize(right=False).
-#include "fq_common.cuh"
+#include "tcgen05.cuh"
 
 namespace fq {
 
@@ -777,11 +779,14 @@ __global__ void __launch_bounds__(kCoopThreads, QJL ? 1 : 2) compress_coop_kerne
 
 }  // namespace fq
 #include "compress_few.cuh"
+#include "compress_tile.cuh"
 namespace fq {
 
-// below this many tiles the CTA-per-tile kernel is the faster one (measured cross-over at
-// about 1000 tiles: it starts in 12 us and needs 6.6 us per wave of tiles, the warp-per-tile
-// kernel 30 us and 33 us per eight tiles and SM)
+// Below this many tiles of 16 vectors the CTA-per-tile kernel is the faster one.  head_dim 64: measured
+// cross-over with the warp-per-tile kernel at about 1000 tiles (it starts in 12 us and needs 6.6 us per wave
+// of tiles, the other 30 us and 33 us per eight tiles and SM).  head_dim 128: as long as every SM has one
+// tile.  us per call against the tcgen05 kernel: 1600 vectors, one source 6.9 / 8.2, keys and values
+// 9.4 / 11.7, two-stage 15.9 / 19.8; 2400 vectors 10.5 / 8.2, 12.1 / 11.8, 22.2 / 19.8.
 constexpr int64_t kCoopMaxTiles = 1024;
 
 template <int D, int DT, bool QJL>
@@ -807,37 +812,51 @@ static int launch_compress_coop(const CompressArgs& a, int64_t tiles, cudaStream
   return check_launch("compress kernel launch");
 }
 
-template <int D, int DT, bool QJL>
-static int launch_compress_t(const CompressArgs& a, cudaStream_t stream) {
-  using S = CompressSmem<D, QJL>;
-  auto kern = compress_kernel<D, DT, QJL>;
+template <int DT, bool QJL>
+static int launch_compress_warp(const CompressArgs& a, int64_t tiles, int sm_count, cudaStream_t stream) {
+  using S = CompressSmem<64, QJL>;
+  auto kern = compress_kernel<64, DT, QJL>;
   static thread_local int configured_device = -1;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(FQ_ERR_CUDA, "cudaGetDevice failed");
-  static thread_local int sm_count = 0;
   if (configured_device != dev) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(S::kBytes));
     if (e != cudaSuccess)
       return fail(FQ_ERR_CUDA, "compress: shared memory opt-in of %zu bytes refused: %s",
                   S::kBytes, cudaGetErrorString(e));
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     configured_device = dev;
   }
+  const int per_sm = QJL ? 1 : 2;
+  const int64_t ctas = (tiles + kCompressWarps - 1) / kCompressWarps;  // a warp per tile
+  const int grid = int(ctas < int64_t(sm_count) * per_sm ? ctas : int64_t(sm_count) * per_sm);
+  kern<<<grid, kCompressThreads, S::kBytes, stream>>>(a);
+  return check_launch("compress kernel launch");
+}
+
+template <int D, int DT, bool QJL>
+static int launch_compress_t(const CompressArgs& a, cudaStream_t stream) {
   const int64_t n_vec = a.n_tokens * a.heads;
   const int64_t tiles = (n_vec + kTileRows - 1) / kTileRows;
   if (tiles == 0) return FQ_OK;
   if (n_vec * a.n_src <= kFewMaxVectors && aligned(a.mat_a, 16) && aligned(a.mat_b, 16) &&
       aligned(a.qjl, 16))
     return launch_compress_few<D, DT, QJL>(a, n_vec, stream);
-  if (tiles < kCoopMaxTiles) return launch_compress_coop<D, DT, QJL>(a, tiles, stream);
+  static thread_local int known_device = -1, sm_count = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fail(FQ_ERR_CUDA, "cudaGetDevice failed");
+  if (known_device != dev) {
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    known_device = dev;
+  }
+  if (tiles <= (D == 128 ? sm_count : kCoopMaxTiles - 1))
+    return launch_compress_coop<D, DT, QJL>(a, tiles, stream);
   FQ_REQUIRE(n_vec < (int64_t(1) << 31) - 16 * 4096, FQ_ERR_UNSUPPORTED,
              "compress: %lld vectors in one call (at most 2^31)", (long long)n_vec);
-  const int per_sm = QJL ? 1 : 2;
-  const int64_t ctas = (tiles + kCompressWarps - 1) / kCompressWarps;  // a warp per tile
-  const int grid = int(ctas < int64_t(sm_count) * per_sm ? ctas : int64_t(sm_count) * per_sm);
-  kern<<<grid, kCompressThreads, S::kBytes, stream>>>(a);
-  return check_launch("compress kernel launch");
+  if constexpr (D == 128)
+    return launch_compress_tile<DT, QJL>(a, n_vec, sm_count, stream);
+  else
+    return launch_compress_warp<DT, QJL>(a, tiles, sm_count, stream);
 }
 
 template <int D, bool QJL>
