@@ -1233,6 +1233,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) paged_decode_kernel(DecodeA
 
 }  // namespace fq
 #include "paged_decode_fast.cuh"
+#include "decode_direct_kernel.cuh"
 namespace fq {
 
 // ------------------------------------------------------------------------------------

@@ -152,22 +152,11 @@ struct FastMid {
   float nk_lo, nk_hi, nv_lo, nv_hi;
 };
 
-// First half of a tile: S^T = K q^T (rows = 16 tokens, columns = (token, head) pairs of the
-// group) and the pairing of the value codes.  After it every register of `r` has been used,
-// so the stage can be given back and `r` refilled for the next tile.
+// S^T = K q^T (rows = 16 tokens, columns = (token, head) pairs of the group).  After it every register
+// of `r` has been used.
 template <bool KPRMT>
-__device__ __forceinline__ void fast_front(const FastWarp& w, const FastRaw& r, uint32_t rows,
-                                           const uint32_t (&qf)[8][2], FastMid& m) {
-  constexpr int HI = fast_row(8);
-  // value codes of tokens 2t, 2t+1, 2t+8, 2t+9, bytes 8g..8g+7 of the head, and the norms of
-  // rows g and g+8: on their way while the key product runs
-  const uint32_t naddr = rows + w.laneN, vaddr = rows + w.laneV;
-  const uint2 x0 = lds64<0>(vaddr), x1 = lds64<kFRowG>(vaddr);
-  const uint2 x2 = lds64<HI>(vaddr), x3 = lds64<HI + kFRowG>(vaddr);
-  m.nk_lo = ldsf<0>(naddr);
-  m.nk_hi = ldsf<HI>(naddr);
-  m.nv_lo = ldsf<544>(naddr);
-  m.nv_hi = ldsf<544 + HI>(naddr);
+__device__ __forceinline__ void fast_keys(const FastWarp& w, const FastRaw& r,
+                                          const uint32_t (&qf)[8][2], FastMid& m) {
   const uint32_t ka[4] = {r.ka.x, r.ka.y, r.ka.z, r.ka.w};
   const uint32_t kb[4] = {r.kb.x, r.kb.y, r.kb.z, r.kb.w};
 #pragma unroll
@@ -200,6 +189,10 @@ __device__ __forceinline__ void fast_front(const FastWarp& w, const FastRaw& r, 
     mma_f16(m.sacc[0], a[0][0], a[0][1], a[0][2], a[0][3], qf[2 * i][0], qf[2 * i][1]);
     mma_f16(m.sacc[1], a[1][0], a[1][1], a[1][2], a[1][3], qf[2 * i + 1][0], qf[2 * i + 1][1]);
   }
+}
+// Value codes of tokens 2t, 2t+1, 2t+8, 2t+9 as table indices.
+__device__ __forceinline__ void fast_pair_values(const uint2 x0, const uint2 x1, const uint2 x2,
+                                                 const uint2 x3, FastMid& m) {
   // even coordinates sit in the high nibbles, odd ones in the low nibbles; equal nibbles of
   // two tokens are paired into one table index
 #pragma unroll
@@ -211,6 +204,25 @@ __device__ __forceinline__ void fast_front(const FastWarp& w, const FastRaw& r, 
     m.ev23[h] = ((c2 >> 4) & 0x0f0f0f0fu) | (c3 & 0xf0f0f0f0u);
     m.od23[h] = (c2 & 0x0f0f0f0fu) | ((c3 << 4) & 0xf0f0f0f0u);
   }
+}
+
+// First half of a tile: the key product and the pairing of the value codes.  After it the stage can be
+// given back and `r` refilled for the next tile.
+template <bool KPRMT>
+__device__ __forceinline__ void fast_front(const FastWarp& w, const FastRaw& r, uint32_t rows,
+                                           const uint32_t (&qf)[8][2], FastMid& m) {
+  constexpr int HI = fast_row(8);
+  // value codes of tokens 2t, 2t+1, 2t+8, 2t+9, bytes 8g..8g+7 of the head, and the norms of
+  // rows g and g+8: on their way while the key product runs
+  const uint32_t naddr = rows + w.laneN, vaddr = rows + w.laneV;
+  const uint2 x0 = lds64<0>(vaddr), x1 = lds64<kFRowG>(vaddr);
+  const uint2 x2 = lds64<HI>(vaddr), x3 = lds64<HI + kFRowG>(vaddr);
+  m.nk_lo = ldsf<0>(naddr);
+  m.nk_hi = ldsf<HI>(naddr);
+  m.nv_lo = ldsf<544>(naddr);
+  m.nv_hi = ldsf<544 + HI>(naddr);
+  fast_keys<KPRMT>(w, r, qf, m);
+  fast_pair_values(x0, x1, x2, x3, m);
 }
 
 // Second half of a tile: online softmax in the accumulator layout, then O^T += V^T P^T.

@@ -34,6 +34,7 @@
 
 #include "fq_common.cuh"
 #include "centroid_scale.cuh"
+#include "decode_direct.cuh"
 #include "tcgen05.cuh"
 
 namespace fq {
@@ -692,6 +693,33 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
     a.out = out;
     rc = attention_prep(a, ws, rotation, rotation_v, stream);
     return rc != FQ_OK ? rc : launch_prefill_pair<false>(a, dtype, stream);
+  }
+  if (n_q == 1 && group <= 8 && rotate_is_few_rows(rows)) {
+    // One query token of up to eight heads per KV head: streamed by warps, a CTA per slice and
+    // (sequence, KV head); the back-rotation merges the slices.  (The query tile below leaves most of
+    // its 128 rows empty on such a call, and needs four launches.)
+    DirectArgs u{};
+    u.q = q; u.rotation = rotation;
+    u.cent_k = centroids_k; u.nck = n_centroids_k;
+    u.cent_v = centroids_v; u.ncv = n_centroids_v;
+    u.seqs = batch; u.hq = num_q_heads; u.hkv = num_kv_heads;
+    u.scale_log2 = a.scale_log2;
+    u.part = reinterpret_cast<float*>(ws + w.part_off);
+    u.status = a.status;
+    u.k_codes = k_packed; u.k_norms = k_norms;
+    u.v_codes = v_packed; u.v_norms = v_norms;
+    u.nkv = n_kv; u.kv_stride = kv_stride;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // one wave of CTAs, and no slice without a tile
+    const int pairs = batch * num_kv_heads, tiles = (n_kv + 15) / 16;
+    const int want = sms / pairs < 1 ? 1 : sms / pairs;
+    u.n_splits = want < kPfMaxSplits ? want : kPfMaxSplits;
+    if (u.n_splits > tiles) u.n_splits = tiles;
+    rc = launch_decode_direct(u, dtype, stream);
+    return rc != FQ_OK ? rc
+                       : rotate_back_merged(u.part, u.n_splits, dtype, rotation_v, out, rows, head_dim, stream);
   }
   {
     // One query token: the query heads of a KV group become the rows of one query tile

@@ -1,0 +1,49 @@
+"""One query token over a contiguous cache, streamed by warps: lengths around the 16-token tiles and the
+slices, one to eight query heads per KV head, byte-permute and look-up keys, buffers with room behind
+the last token."""
+
+import math
+
+import pytest
+import torch
+
+import flashquant_b200 as fq
+from oracle import tq_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("hq,hkv", [(1, 1), (6, 2), (8, 2), (16, 2), (32, 8), (64, 64)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 255, 273, 4099])
+@pytest.mark.parametrize("k_bits,dtype", [(3, torch.float16), (4, torch.bfloat16)])
+def test_one_token(consts, hq, hkv, n, k_bits, dtype):
+    if hkv == 64 and n > 1000:
+        pytest.skip("more than one wave of CTAs is covered by the short ones")
+    b, d, cap = 3, 128, n + 5
+    rot_k, rot_v = consts["rotation_128_0"], fq.haar_orthogonal(d, seed=43)
+    bk, ck = consts[f"boundaries_128_{k_bits}"], consts[f"centroids_128_{k_bits}"]
+    bv, cv = consts["boundaries_128_4"], consts["centroids_128_4"]
+    g = torch.Generator().manual_seed(100 * n + hq)
+    k, v = torch.randn(2, b, hkv, n, d, generator=g)
+    k[..., 9] *= 10.0
+    q = torch.randn(b, hq, 1, d, generator=g).to(dtype)
+    bufs, deq = [], []
+    for x, r, bnd, c in ((k, rot_k, bk, ck), (v, rot_v, bv, cv)):
+        p, nm = O.compress(x.reshape(-1, d), r, bnd)
+        deq.append((c.double()[O.nibble_unpack(p).long()] * nm.reshape(-1, 1).double()).view(b, hkv, n, d))
+        codes = torch.full((b, hkv, cap, d // 2), 255, dtype=torch.uint8)
+        norms = torch.full((b, hkv, cap, 1), math.nan)  # nothing behind the last token counts
+        codes[:, :, :n] = p.view(b, hkv, n, -1)
+        norms[:, :, :n] = nm.view(b, hkv, n, 1)
+        bufs += [codes.to(DEV)[:, :, :n], norms.to(DEV)[:, :, :n]]
+    got = fq.fused_tq_attention_kv(q.to(DEV), *bufs, ck, cv, rot_k, rot_v)
+    # the rotated query is rounded to its type, everything else in 64 bits
+    q_rot = (q.double() @ rot_k.double().T).to(dtype).double().view(b, hkv, hq // hkv, d)
+    s = torch.softmax(q_rot @ deq[0].transpose(-1, -2) / math.sqrt(d), dim=-1)
+    ref = ((s @ deq[1]) @ rot_v.double()).view(b, hq, 1, d)
+    # one rounding of the result (2^-8 or 2^-11 of an entry; its rms is about half of that) and fp16
+    # tables and weights (2^-11 at most)
+    rel = ((got.cpu().double() - ref).norm() / ref.norm()).item()
+    bound = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10}[dtype]
+    assert rel <= bound, rel
