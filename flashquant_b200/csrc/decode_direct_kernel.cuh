@@ -7,6 +7,9 @@
 // first tiles are on their way meanwhile, a warp reads its tiles from memory straight into registers one
 // tile ahead (a head's 16 tokens are 1 KB of consecutive bytes: nothing to stage), the 16 warps merge in
 // shared memory, and the launch that rotates back merges the slices.
+//
+// Measured, attention call, against the 128-row query tile (32 / 8 heads): 1 x 20 tokens 22 -> 14 us, 4 x 4000
+// 48 -> 20 us, 8 x 16384 220 -> 56 us (2.5 TB/s; one dependent chain per warp and tile bounds it).
 #pragma once
 
 #include "decode_direct.cuh"

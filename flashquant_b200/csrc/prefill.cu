@@ -2,7 +2,8 @@
 //
 // Two kernels: prefill_pair_kernel (prefill_pair.cuh) for calls with many query rows, contiguous
 // or paged, and prefill_attention_kernel below for one query token per sequence over a contiguous
-// cache, whose keys are cut into slices so that the CTAs fill the GPU.
+// cache with more than eight query heads per KV head or more than
+// 1024 rows (other single tokens: decode_direct_kernel).
 //
 // prefill_attention_kernel: one CTA of 256 threads owns the query rows of one (batch, KV head) - two
 // threads per row, each with half of the columns - and walks its slice in tiles of 64 tokens.
