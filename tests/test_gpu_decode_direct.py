@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("hq,hkv", [(1, 1), (6, 2), (8, 2), (16, 2), (32, 8), (64, 64)])
+@pytest.mark.parametrize("hq,hkv", [(6, 2), (8, 2), (16, 2), (32, 8), (64, 64)])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 255, 273, 4099])
 @pytest.mark.parametrize("k_bits,dtype", [(3, torch.float16), (4, torch.bfloat16)])
 def test_one_token(consts, hq, hkv, n, k_bits, dtype):
