@@ -70,7 +70,7 @@ constexpr int kMaxChunkJobs = 1024;
 constexpr uint32_t kMergeScratchBytes =
     (kMergeHeads * 128 + kMergeHeads * kComputeThreads / 2 + 64 + kMaxParts + 4) * 4;
 
-enum : int { kSegStart = 1, kSegEnd = 2, kQNew = 4 };
+enum : int { kSegStart = 1, kSegEnd = 2, kQNew = 4, kQLast = 8 };
 
 struct DecodeArgs {
   const __half* q_rot;  // (num_seqs, Hq, D)
@@ -767,7 +767,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) paged_decode_kernel(DecodeA
       int n_valid = p.seq_lens[seq] - pg * p.block_size;  // pg < max_pages: see the prefix
       if (n_valid > p.block_size) n_valid = p.block_size;
       const int flags =
-          (seg_first ? kSegStart : 0) | (seg_last ? kSegEnd : 0) | (q_new ? kQNew : 0);
+          (seg_first ? kSegStart : 0) | (seg_last ? kSegEnd : 0) | (q_new ? kQNew : 0) |
+          (pg + 1 == n_pages ? kQLast : 0);
       ring[i & (kDescRing - 1)] =
           make_int4(int(phys), n_valid | (flags << 8), seq, seq * p.num_splits + s + int(wk));
     };
@@ -983,10 +984,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) paged_decode_kernel(DecodeA
           qf[s][1] = valid ? v.y : 0u;
         }
         // the loads must have delivered before the buffer goes back to the producer: a load in
-        // flight is not ordered before the arrive by anything else
-        __threadfence_block();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(qempty_bar);
+        // flight is not ordered before the arrive by anything else.  (With QS the buffer's second
+        // half, q S^T, is read for every page: it goes back after the sequence's last one.)
+        if constexpr (!QS) {
+          __threadfence_block();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(qempty_bar);
+        }
         ++qcnt;
       }
     }
@@ -1220,7 +1224,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) paged_decode_kernel(DecodeA
 
     __threadfence_block();  // as for the query buffer: loads from the stage delivered, then release
     __syncwarp();
-    if (lane == 0) mbar_arrive(empty_bar + stage);
+    if (lane == 0) {
+      mbar_arrive(empty_bar + stage);
+      if (QS && (flags & kQLast)) mbar_arrive(qempty_bar);
+    }
     if (++stage == stages) { stage = 0; fphase ^= 1; }
   }
   if (timed_out && lane == 0) atomicOr(p.status, FQ_DEV_WAIT_TIMEOUT);

@@ -5,6 +5,8 @@ agree within 2e-3 max-abs and 2^-10 of the entry; after both roundings an entry 
 one unit in its last place plus the rounding flips the reference's own values allow.
 """
 
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -462,6 +464,57 @@ def test_two_stage_scoring_vs_oracle(consts, dtype):
     assert (plain.float() - out.float()).abs().max().item() > 1e-2
     ws = K.decode_workspace(torch.device(DEV), w.num_seqs, hq, hkv, d, 0)
     assert K.workspace_status(ws) == 0
+
+
+@pytest.mark.parametrize("hq,hkv,seqs,longest", [(16, 2, 98, 600), (32, 8, 40, 300), (8, 1, 150, 90)])
+def test_two_stage_many_sequences_per_team(consts, hq, hkv, seqs, longest):
+    """Teams whose runs cover several sequences: q S^T of a sequence stays in the team's buffer until
+    its last page has been scored.  Rows against the estimator in 64 bits, and the same bits each time."""
+    d, bs, dtype = 128, 16, torch.float16
+    rot, S = consts["rotation_128_0"], consts["qjl_128_0"]
+    bk, ck = consts["boundaries_128_3"], consts["centroids_128_3"]
+    bv, cv = consts["boundaries_128_4"], consts["centroids_128_4"]
+    g = torch.Generator().manual_seed(seqs)
+    lens = torch.randint(longest // 4, longest + 1, (seqs,), generator=g).tolist()
+    w = W.decode_workload(num_q_heads=hq, num_kv_heads=hkv, head_dim=d, block_size=bs, cfg=3,
+                          seq_lens=lens, dtype=dtype)
+    k, v = W.make_kv(w.total_tokens, hkv, d, 3, dtype)
+    cache = torch.zeros(w.num_blocks, bs, hkv * (d + 8), dtype=torch.uint8, device=DEV)
+    plane = torch.zeros(w.num_blocks, bs, hkv * (d // 8 + 4), dtype=torch.uint8, device=DEV)
+    K.tq4_compress_append_qjl(k.to(DEV), v.to(DEV), cache, plane, w.slot_mapping.to(DEV), rot, bk,
+                              ck, bv, S)
+    args = (w.q.to(DEV), cache, plane, w.block_table.to(DEV), w.seq_lens.to(DEV), ck, cv, rot, S,
+            hkv, d, bs)
+    out = K.split_k_paged_decode_qjl(*args)
+    for _ in range(10):
+        assert torch.equal(K.split_k_paged_decode_qjl(*args), out)
+    # 64 bits, from the stored bytes; the rotated query is rounded to its type
+    slots = w.slot_mapping.to(DEV)
+    rows = cache.view(-1, hkv * (d + 8))[slots]
+    prow = plane.view(-1, hkv * (d // 8 + 4))[slots]
+    at, n, half = 0, hkv * d // 2, hkv * d // 8
+    f64 = {n_: t.to(DEV).double() for n_, t in dict(rot=rot, S=S, ck=ck, cv=cv).items()}
+    bit = torch.arange(8, device=DEV, dtype=torch.uint8)
+    worst = 0.0
+    for i, length in enumerate(lens):
+        r, p = rows[at:at + length], prow[at:at + length]
+        at += length
+        un = lambda x: torch.stack((x >> 4, x & 15), -1).flatten(-2).long().view(length, hkv, d)
+        norm = lambda x: x.contiguous().view(torch.float32).double().unsqueeze(-1)
+        keys = f64["ck"][un(r[:, :n])] * norm(r[:, n:n + 4 * hkv])
+        vals = f64["cv"][un(r[:, n + 4 * hkv:2 * n + 4 * hkv])] * norm(r[:, 2 * n + 4 * hkv:])
+        signs = ((p[:, :half].unsqueeze(-1) >> bit) & 1).view(length, hkv, d).double() * 2 - 1
+        q = w.q[i].to(DEV).double().view(hkv, hq // hkv, d)
+        s = torch.einsum("hgd,lhd->hgl", (q @ f64["rot"].T).to(dtype).double(), keys)
+        s += torch.einsum("hgd,lhd->hgl", q @ f64["S"].T, signs * norm(p[:, half:])) * \
+            math.sqrt(math.pi / 2) / d
+        o = torch.einsum("hgl,lhd->hgd", torch.softmax(s / math.sqrt(d), -1), vals) @ f64["rot"]
+        o = o.reshape(hq, d)
+        worst = max(worst, ((out[i].double() - o).norm(dim=-1) / o.norm(dim=-1)).max().item())
+    # two roundings to fp16 of the row, fp16 tables and weights, and q S^T in fp16: the last makes a
+    # logit's error about 2^-11 of the correction term (|.| < 10), 2^-8 of a weight
+    assert worst <= 2.0 ** -7, worst
+    assert K.workspace_status(K.decode_workspace(torch.device(DEV), seqs, hq, hkv, d, 0)) == 0
 
 
 def test_three_launch_form_gives_the_same_answer(consts):
