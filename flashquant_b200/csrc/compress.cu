@@ -778,6 +778,7 @@ __global__ void __launch_bounds__(kCoopThreads, QJL ? 1 : 2) compress_coop_kerne
 }
 
 }  // namespace fq
+#include "compress_recheck.cuh"
 #include "compress_few.cuh"
 #include "compress_tile.cuh"
 namespace fq {

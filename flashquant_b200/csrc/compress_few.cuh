@@ -14,10 +14,12 @@
 namespace fq {
 
 constexpr int kFewVecs = 4;
-// Above this the CTA-per-tile kernel is faster: every CTA reads the 64 KB of its matrix from the L2.
-// Kernel time in us, keys and values of n tokens x 8 heads (the CTA-per-tile kernel in brackets):
-// n = 1: 4.0 (6.7), 32: 4.2 (7.2), 73: 5.4 (7.3); two-stage 6.2 (12.9), 6.4 (13.6), 9.5 (13.9).
-constexpr int64_t kFewMaxVectors = 1600;
+// One wave: two CTAs on each of 148 SMs.  Above it the CTA-per-tile kernel is faster, as every CTA reads the
+// 64 KB of its matrix from the L2.  Time per call in us, keys and values of n tokens x 8 heads (the
+// CTA-per-tile kernel in brackets): n = 1: 3.8 (6.8), 32: 4.9 (7.5), 73: 6.7 (7.6), 100: 8.8 (7.6); two-stage
+// 6.4 (13.2), 8.5 (14.1), 12.0 (14.2), 15.8 (14.2); head_dim 64 3.2 (4.7), 3.7 (5.2), 3.9 (5.2), 4.5 (5.3).
+// (The recheck is about 0.7 us of 32 tokens and 1.3 us of 73: some CTA of the call has one.)
+constexpr int64_t kFewMaxVectors = 1184;
 
 template <int D, int DT, bool kTwoStage>
 __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
@@ -27,6 +29,8 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
   constexpr int kLenA = D / 32, kLenB = D / 16, kQuads = D / 4;
   constexpr int kWarpsPerVec = D / 32;
   __shared__ __align__(16) float xs[kFewVecs][D];
+  __shared__ __align__(16) float xr[kFewVecs][D];  // the vectors as they came
+  __shared__ float s_nrm[kFewVecs];
   __shared__ __align__(16) float red[16][kFewVecs][D];
   __shared__ float part[kThreads / 32];
   __shared__ float s_bnd[16], s_cent[16];
@@ -162,19 +166,53 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
     return sum;
   };
 
-  // ---- norm, x_hat -------------------------------------------------------------------------------
-  const float nrm = sqrtf(vector_sum(x * x));
+  // ---- norm (summed as compress_coop_kernel does), x_hat ------------------------------------------
+  xr[r][j] = x;
+  __syncthreads();
+  float ss = 0.f;
+#pragma unroll
+  for (int q = 0; q < kLenA; ++q) ss = fmaf(xr[r][lane * kLenA + q], xr[r][lane * kLenA + q], ss);
+  const float nrm = sqrtf(warp_sum(ss));
   xs[r][j] = x * (1.f / (nrm + 1e-10f));
-  if (j == 0 && slot_r >= 0)
-    *reinterpret_cast<float*>(p.norm[s] + slot_r * p.norm_row_stride + head_r * 4) = nrm;
+  if (j == 0) {
+    s_nrm[r] = nrm;
+    if (slot_r >= 0)
+      *reinterpret_cast<float*>(p.norm[s] + slot_r * p.norm_row_stride + head_r * 4) = nrm;
+  }
   __syncthreads();
 
   // ---- y = x_hat Pi^T, codes; the centroid vector replaces x_hat --------------------------------
   int idx;
+  float y;
   if (p.rot_split) {
     product_cols(fwd);
     __syncthreads();
-    idx = bucketize15(gather((j >> 1) + (j & 1) * (D / 2)), s_bnd);
+    y = gather((j >> 1) + (j & 1) * (D / 2));
+  } else {
+    y = product_rows(fwd);
+  }
+  idx = bucketize15(y, s_bnd);
+  // (a zero vector's coordinates are zero in any arithmetic)
+  const bool near = near_boundary(y, idx, s_bnd) && s_nrm[p.rot_split ? r : sl] > 0.f;
+  if (const uint32_t lanes = __ballot_sync(0xffffffffu, near)) {
+    if (p.rot_split) {
+      const int col0 = j - lane;  // the warp's 32 columns of vector r, eight at a time
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        if (!(lanes >> (8 * c) & 0xffu)) continue;
+        const float2 f = recheck_columns<D, kMatSplit>(xs[r], 1, mat_a, mat_b, col0 + 8 * c);
+        const float f0 = __shfl_sync(0xffffffffu, f.x, (lane & 7) >> 1);
+        const float f1 = __shfl_sync(0xffffffffu, f.y, (lane & 7) >> 1);
+        if (lane >> 3 == c) idx = bucketize15((lane & 1) ? f1 : f0, s_bnd);
+      }
+    } else {
+      const float2 f = recheck_columns<D, kMatRows>(xs[0], kFewVecs, mat_a, nullptr, 8 * warp);
+      const float f0 = __shfl_sync(0xffffffffu, f.x, 4 * sl + (lane >> 3));
+      const float f1 = __shfl_sync(0xffffffffu, f.y, 4 * sl + (lane >> 3));
+      idx = bucketize15((lane >> 2 & 1) ? f1 : f0, s_bnd);
+    }
+  }
+  if (p.rot_split) {
     // a warp holds 32 consecutive columns of vector r: eight lanes make a word
     uint32_t w = uint32_t(idx) << (8 * ((j >> 1) & 3) + ((j & 1) ? 0 : 4));
     w |= __shfl_xor_sync(0xffffffffu, w, 1);
@@ -184,7 +222,6 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
       *reinterpret_cast<uint32_t*>(p.code[s] + slot_r * p.code_row_stride +
                                    int64_t(head_r) * p.code_head_stride + j / 2) = w;
   } else {
-    idx = bucketize15(product_rows(fwd), s_bnd);
     // a warp holds columns 8*warp .. 8*warp+7 of every vector, column = lane / 4
     uint32_t w = uint32_t(idx) << (8 * (lane >> 3) + ((ja & 1) ? 0 : 4));
     w |= __shfl_xor_sync(0xffffffffu, w, 4);
@@ -211,10 +248,27 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
     if (j == 0 && slot_r >= 0)
       *reinterpret_cast<float*>(p.gam + slot_r * p.gam_row_stride + head_r * 4) = gam;
     // ---- sign(r S^T): bit j%8 of byte j/8 is 1 for a projection >= 0; a warp makes one byte ------
-    uint32_t b = product_rows(sgn) >= 0.f ? 1u << (lane >> 2) : 0u;
+    const float proj = product_rows(sgn);
+    uint32_t b = proj >= 0.f ? 1u << (lane >> 2) : 0u;
     b |= __shfl_xor_sync(0xffffffffu, b, 4);
     b |= __shfl_xor_sync(0xffffffffu, b, 8);
     b |= __shfl_xor_sync(0xffffffffu, b, 16);
+    if (__syncthreads_or(fabsf(proj) <= kNearZero * s_nrm[sl] && s_nrm[sl] > 0.f)) {
+      // the chain from the codes on, eight columns a warp (the residual has been read)
+      const int g = lane >> 2, col = 8 * warp + 2 * (lane & 3);
+      xs[sl][ja] = s_cent[idx];
+      __syncthreads();
+      float2 f = recheck_columns<D, kMatCols>(&xs[0][0], kFewVecs, p.mat_a, nullptr, 8 * warp);
+      if (g < kFewVecs)
+        *reinterpret_cast<float2*>(&red[0][g][col]) =
+            make_float2(fmaf(-f.x, s_nrm[g], xr[g][col]), fmaf(-f.y, s_nrm[g], xr[g][col + 1]));
+      __syncthreads();
+      f = recheck_columns<D, kMatRows>(&red[0][0][0], kFewVecs, p.qjl, nullptr, 8 * warp);
+      b = ((f.x >= 0.f ? 1u : 0u) | (f.y >= 0.f ? 2u : 0u)) << (2 * (lane & 3));
+      b |= __shfl_xor_sync(0xffffffffu, b, 1);
+      b |= __shfl_xor_sync(0xffffffffu, b, 2);
+      b = __shfl_sync(0xffffffffu, b, 4 * (lane & 3));  // lane i < 4: of vector i
+    }
     if (lane < 4 && slot_sl >= 0)
       p.sign[slot_sl * p.sign_row_stride + head_sl * (D / 8) + warp] = uint8_t(b);
   }
