@@ -9,7 +9,7 @@
 // either side with any summation order) at a third of the multiply-add issue slots of an fp32
 // FMA contraction, which was the bound of this kernel before.
 //
-// Four kernels by number of vectors: a few (compress_few.cuh), up to a tile of 16 per SM
+// Four kernels by number of vectors: a few (compress_few.cuh), up to two tiles of 16 per SM
 // (compress_coop_kernel), many of head_dim 128 (compress_tile.cuh: tcgen05) and many of head_dim 64:
 // compress_kernel, a CTA of 8 warps that keeps the matrices resident in shared memory as fp16 hi / lo' planes (the
 // same bytes as fp32).  A warp owns a tile of 16 vectors end to end, K of the tile then V:
@@ -60,6 +60,7 @@ struct CompressArgs {
   // source 1 by another rotation (null: mat_a / mat_b); compress_few_kernel only
   const float* mat_a1;
   const float* mat_b1;
+  int sum_by_quads;  // order of the sum of squares (compress_tile_kernel): as compress_kernel's
 };
 
 __device__ __forceinline__ int64_t segment_row(const CompressArgs& p, uint32_t tok) {
@@ -89,6 +90,16 @@ __device__ __forceinline__ void split_hi_lo(float v, __half& hi, __half& lo) {
 }
 __device__ __forceinline__ uint32_t pack_h2(__half a, __half b) {
   return uint32_t(__half_as_ushort(a)) | (uint32_t(__half_as_ushort(b)) << 16);
+}
+
+// Four code bytes; a caller's buffer of codes need only be aligned to two.
+__device__ __forceinline__ void store_code_word(uint8_t* dst, uint32_t w) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+    *reinterpret_cast<uint32_t*>(dst) = w;
+  } else {
+    reinterpret_cast<uint16_t*>(dst)[0] = uint16_t(w);
+    reinterpret_cast<uint16_t*>(dst)[1] = uint16_t(w >> 16);
+  }
 }
 
 // index = #{b : b < y} over an ascending table padded with +inf to 15 entries
@@ -129,10 +140,13 @@ __device__ __forceinline__ void stage_matrix(__half* hi, __half* lo, int ld, boo
   }
 }
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* row_ptr) {
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t row) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(row_ptr)));
+               : "r"(row));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* row_ptr) {
+  ldmatrix_x4(r, smem_u32(row_ptr));
 }
 
 // One product of a 16-row tile held in registers with a resident matrix, four column tiles at
@@ -785,9 +799,10 @@ namespace fq {
 
 // Below this many tiles of 16 vectors the CTA-per-tile kernel is the faster one.  head_dim 64: measured
 // cross-over with the warp-per-tile kernel at about 1000 tiles (it starts in 12 us and needs 6.6 us per wave
-// of tiles, the other 30 us and 33 us per eight tiles and SM).  head_dim 128: as long as every SM has one
-// tile.  us per call against the tcgen05 kernel: 1600 vectors, one source 6.9 / 8.2, keys and values
-// 9.4 / 11.7, two-stage 15.9 / 19.8; 2400 vectors 10.5 / 8.2, 12.1 / 11.8, 22.2 / 19.8.
+// of tiles, the other 30 us and 33 us per eight tiles and SM).  head_dim 128: as long as no SM has more than two
+// tiles.  us per call against the tcgen05 kernel: 2400 vectors, one source 11.0 / 11.5, keys and values
+// 10.7 / 12.8, two-stage 20.4 / 22.7; 4720 vectors 11.2 / 11.6, 10.8 / 13.1, 20.9 / 23.0; 5600 vectors
+// 11.8 / 11.6, 13.5 / 13.1, 27.1 / 23.1.
 constexpr int64_t kCoopMaxTiles = 1024;
 
 template <int D, int DT, bool QJL>
@@ -850,12 +865,12 @@ static int launch_compress_t(const CompressArgs& a, cudaStream_t stream) {
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     known_device = dev;
   }
-  if (tiles <= (D == 128 ? sm_count : kCoopMaxTiles - 1))
+  if (tiles <= (D == 128 ? 2 * sm_count : kCoopMaxTiles - 1))
     return launch_compress_coop<D, DT, QJL>(a, tiles, stream);
   FQ_REQUIRE(n_vec < (int64_t(1) << 31) - 16 * 4096, FQ_ERR_UNSUPPORTED,
              "compress: %lld vectors in one call (at most 2^31)", (long long)n_vec);
   if constexpr (D == 128)
-    return launch_compress_tile<DT, QJL>(a, n_vec, sm_count, stream);
+    return launch_compress_tile<DT, QJL>(a, n_vec, tiles >= kCoopMaxTiles, sm_count, stream);
   else
     return launch_compress_warp<DT, QJL>(a, tiles, sm_count, stream);
 }

@@ -1,6 +1,6 @@
 // Many vectors of head_dim 128: the products on tcgen05 with 128-vector tiles.  Included by compress.cu.
 //
-// The element-wise work around the products bounds the compressor (about 22 instructions per
+// The element-wise work around the products bounds the compressor (about 28 instructions per
 // coordinate: split into fp16 terms, bucketize, pack), and the warp-per-tile kernel could not overlap it
 // with its own `mma.sync` chain: 8 warps per SM, tensor pipe 35 % busy.  Here the products leave the
 // warps altogether.  A CTA of 512 threads is two groups of 256; a group owns a tile of 128
@@ -13,10 +13,13 @@
 // the other kernels: hi lo' + lo' hi is accumulated first, and the first hi hi MMA scales that sum by 2^-11
 // (scale-input-d), so one accumulator does.
 //
-// Measured (per call): 8192 tokens x 8 heads, two-stage keys: 144 -> 56 us; 262 144 vectors of one source
-// 124 -> 56 us (1.5 TB/s); 8000 vectors 13.3 -> 8.3 us.  At 262 144 vectors the schedulers issue in 46 % of
-// the cycles (27 M warp instructions); the rest is the two groups meeting in the same phase, and the 32
-// lines that every 16-byte load of a row per thread touches (load/store wavefronts 51 % of peak).
+// Codes and signs next to a decision are left to the arithmetic of the 16-row kernels (compress_recheck.cuh): a
+// group notes such vectors and computes them again, 16 at a time, when its items are done.  (As a
+// call inside the loop it cost 24 us of 262 144 vectors in spilled registers.)
+//
+// Measured (per call): 8192 tokens x 8 heads, two-stage keys: 143 -> 63 us; 262 144 vectors of one source
+// 127 -> 69 us (1.3 TB/s); 8000 vectors 14 -> 11.7 us.  Of the 69 us the order of the sum of squares takes 2,
+// the distances to the boundaries 5, the recheck 3.  Two-stage fp32 input spills 32 bytes.
 #pragma once
 
 namespace fq {
@@ -26,6 +29,9 @@ constexpr int kTileGroup = 256;
 constexpr int kTileVecs = 128;
 constexpr uint32_t kTileSlab = 128 * 16;        // one 8-element k chunk of 128 matrix rows
 constexpr uint32_t kTilePlane = 128 * 128 * 2;  // one fp16 plane of a matrix, [k chunk][row][16 B]
+constexpr int kTileLd = 128 + 8;                // halves per row of a recheck's left operand
+constexpr uint32_t kTileXch = 2 * 16 * kTileLd * 2;
+constexpr int kTileList = 512;   // vectors a group can note; if there are more, it rechecks all of its own
 
 template <bool QJL>
 struct TileSmem {
@@ -33,12 +39,21 @@ struct TileSmem {
   static constexpr uint32_t kBnd = kMats * 2 * kTilePlane;  // [2][16] f32
   static constexpr uint32_t kCent = kBnd + 32 * 4;          // [16] hi | lo' << 16
   static constexpr uint32_t kPart = kCent + 16 * 4;         // [2 groups][|x|^2, gamma^2][2 halves][128]
-  static constexpr uint32_t kBar = kPart + 2 * 2 * 2 * 128 * 4;
+  // per group: [16][128] partial sums of |x|^2; in a recheck the left operand's hi and lo' rows
+  static constexpr uint32_t kXch = kPart + 2 * 2 * 2 * 128 * 4;
+  static constexpr uint32_t kList = kXch + 2 * kTileXch;  // [2 groups][kTileList] vectors noted for a recheck
+  static constexpr uint32_t kBar = kList + 2 * kTileList * 8;
   static constexpr uint32_t kBytes = kBar + 32;
 };
+static_assert(TileSmem<true>::kBytes <= 227 * 1024, "shared memory of one CTA");
 
 __device__ __forceinline__ void group_sync(int group) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kTileGroup) : "memory");
+}
+__device__ __forceinline__ float min_abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
@@ -103,6 +118,17 @@ struct TileRaw {
       return f2_pack(f.x, f.y);
     }
   }
+  // the same, not to be kept unpacked for a later use of pair(i) (64 registers)
+  __device__ __forceinline__ float2 once(int i) const {
+    TileRaw r;
+    constexpr int kPer = DT == FQ_F32 ? 2 : 1;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      r.w[k] = w[kPer * i + k];
+      if constexpr (DT != FQ_F32) asm volatile("" : "+r"(r.w[k]));
+    }
+    return f2_unpack(r.pair(0));
+  }
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < kWords; ++i) w[i] = 0u;
@@ -125,15 +151,23 @@ struct TileRaw {
   }
 };
 
-// 4 * index of y in the boundary table at `sb`; b3, b7, b11 are the table's entries
+// 4 * index of y in the boundary table at `sb`; b3, b7, b11 are the table's entries.  `least`: smallest
+// distance to a boundary (the two around y are among the four it is compared with)
 __device__ __forceinline__ uint32_t bucket_offset(float y, const unsigned char* sb, float b3, float b7,
-                                                  float b11) {
-  const bool up = y > b7;
-  uint32_t off = up ? 32u : 0u;
-  off += y > (up ? b11 : b3) ? 16u : 0u;
-  off += y > *reinterpret_cast<const float*>(sb + off + 4) ? 8u : 0u;
-  off += y > *reinterpret_cast<const float*>(sb + off) ? 4u : 0u;
+                                                  float b11, float& least) {
+  const float d7 = y - b7, d3 = y - (d7 > 0.f ? b11 : b3);
+  uint32_t off = d7 > 0.f ? 32u : 0u;
+  off += d3 > 0.f ? 16u : 0u;
+  const float d1 = y - *reinterpret_cast<const float*>(sb + off + 4);
+  off += d1 > 0.f ? 8u : 0u;
+  const float d0 = y - *reinterpret_cast<const float*>(sb + off);
+  off += d0 > 0.f ? 4u : 0u;
+  least = min_abs(min_abs(least, d7, d3), d1, d0);
   return off;
+}
+// code byte of two offsets: even coordinate << 4 | odd coordinate
+__device__ __forceinline__ uint32_t code_byte(uint32_t even, uint32_t odd) {
+  return (even << 2) | (odd >> 2);
 }
 
 // Stage a matrix as hi / lo' operand planes, plane[n][k] = get(n, k).  kRows: a row is contiguous in k, so a
@@ -192,6 +226,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
   if constexpr (DT != FQ_F32)
     wide = (p.token_stride & 7) == 0 && ((reinterpret_cast<uintptr_t>(p.src[0]) |
                                           reinterpret_cast<uintptr_t>(p.src[p.n_src - 1])) & 15) == 0;
+  // row that token tok goes to, below 0 for none
+  auto row_of = [&](uint32_t tok) -> int64_t {
+    if (!p.slots) return p.seg_len ? segment_row(p, tok) : int64_t(tok);
+    const int64_t slot = p.slot64 ? reinterpret_cast<const int64_t*>(p.slots)[tok]
+                                  : int64_t(reinterpret_cast<const int32_t*>(p.slots)[tok]);
+    return slot < p.num_slots ? slot : -1;
+  };
   // the thread's vector of work item `it`
   TileRaw<DT> raw;
   int64_t slot = -1;
@@ -209,13 +250,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
     head = int(vec - tok * heads);
     raw.load(static_cast<const T*>(p.src[s]) + int64_t(tok) * p.token_stride + head * D + 64 * half,
              wide);
-    if (p.slots) {
-      slot = p.slot64 ? reinterpret_cast<const int64_t*>(p.slots)[tok]
-                      : int64_t(reinterpret_cast<const int32_t*>(p.slots)[tok]);
-      if (slot >= p.num_slots) slot = -1;
-    } else {
-      slot = p.seg_len ? segment_row(p, tok) : int64_t(tok);
-    }
+    slot = row_of(tok);
   };
   fetch(item);  // on its way while the matrices are laid out
 
@@ -225,6 +260,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
     mbar_init(bars + 1, 1);
     mbar_fence_init();
   }
+  if (tid < 2) reinterpret_cast<uint32_t*>(smem + S::kBar + 20)[tid] = 0;
   if (p.rot_split) {
     stage_planes<false>(smem, tid, [&](int n, int k0, float (&v)[8]) {
       const float* src = ((n & 1) ? p.mat_b : p.mat_a) + k0 * (D / 2) + (n >> 1);
@@ -267,6 +303,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
   const uint32_t a_mine = a_tmem + lane_base + 32 * half;
   const uint32_t planes = smem_u32(smem);
   float* part = reinterpret_cast<float*>(smem + S::kPart) + group * 512 + row;
+  float* xch = reinterpret_cast<float*>(smem + S::kXch + group * kTileXch) + row;
+  uint2* list = reinterpret_cast<uint2*>(smem + S::kList) + group * kTileList;  // vector | source << 31, |x|
+  uint32_t* listed = reinterpret_cast<uint32_t*>(smem + S::kBar + 20) + group;
   uint64_t* bar = bars + group;
   uint32_t parity = 0;
   bool dead = false;
@@ -291,6 +330,178 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
     tc_fence_after();
   };
 
+  // This row of the item, if `near`: into the list.
+  auto note = [&](bool near, int s, float nrm) {
+    const uint32_t rows = __ballot_sync(0xffffffffu, near);
+    if (rows == 0) return;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(listed, uint32_t(__popc(rows)));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(rows & ((1u << lane) - 1));
+    if (near && at < kTileList) {
+      const uint32_t vec = (item - (s ? n_tiles : 0u)) * kTileVecs + row;
+      list[at] = make_uint2(vec | uint32_t(s) << 31, __float_as_uint(nrm));
+    }
+  };
+  // The group's list, 16 vectors at a time, by the arithmetic of compress_coop_kernel: a warp has 16 columns.
+  auto work_off = [&]() {
+    group_sync(group);
+    uint32_t n = *const_cast<volatile uint32_t*>(listed);
+    const uint32_t first = blockIdx.x + uint32_t(group) * gridDim.x;
+    const bool all = n > kTileList;
+    if (all) n = (n_items - first + stride - 1) / stride * kTileVecs;
+    const int wg = warp & 7, g = lane >> 2, t = lane & 3;
+    const int j = lane >> 3, r8 = lane & 7;  // ldmatrix: lanes 8j .. give the rows of matrix j
+    __half* a_hi = reinterpret_cast<__half*>(smem + S::kXch + group * kTileXch);
+    __half* a_lo = a_hi + 16 * kTileLd;
+    float* gpart = reinterpret_cast<float*>(smem + S::kPart) + group * 512;  // [8 warps][16]
+    const uint32_t a_lane = smem_u32(a_hi + ((j & 1) * 8 + r8) * kTileLd + 8 * (j >> 1));
+    const uint32_t b_lane = planes + (j >> 1) * kTilePlane + (j & 1) * kTileSlab + (16 * wg + r8) * 16;
+    auto chain = [&](int m, float(&acc)[2][4]) {
+      float hi[2][4] = {}, co[2][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t xh[4], xl[4], b[4];
+        ldmatrix_x4(xh, a_lane + 32 * ks);
+        ldmatrix_x4(xl, a_lane + 32 * kTileLd + 32 * ks);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          ldmatrix_x4(b, b_lane + m * 2 * kTilePlane + 2 * ks * kTileSlab + i * 128);
+          mma_f16(hi[i], xh[0], xh[1], xh[2], xh[3], b[0], b[1]);
+          mma_f16(co[i], xh[0], xh[1], xh[2], xh[3], b[2], b[3]);
+          mma_f16(co[i], xl[0], xl[1], xl[2], xl[3], b[0], b[1]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(co[i][c], kLoUnscale, hi[i][c]);
+    };
+    // entry e of the list (zeros beyond the last): source, its vector's elements, destination row and head
+    struct Entry {
+      int s, head;
+      float nrm;
+      const T* x;
+      int64_t slot;
+    };
+    auto entry = [&](uint32_t e) {
+      Entry v{0, 0, 0.f, nullptr, -1};
+      if (e >= n) return v;
+      uint32_t vec;
+      if (all) {
+        const uint32_t it = first + e / kTileVecs * stride;
+        v.s = it >= n_tiles;
+        vec = (v.s ? it - n_tiles : it) * kTileVecs + e % kTileVecs;
+        if (vec >= n_vec) return v;
+      } else {
+        const uint2 w = list[e];
+        v.s = int(w.x >> 31);
+        vec = w.x & 0x7fffffffu;
+        v.nrm = __uint_as_float(w.y);
+      }
+      const uint32_t tok = vec / heads;
+      v.slot = row_of(tok);
+      if (v.slot < 0) return v;
+      v.head = int(vec - tok * heads);
+      if (all) v.nrm = *reinterpret_cast<const float*>(p.norm[v.s] + v.slot * p.norm_row_stride + v.head * 4);
+      v.x = static_cast<const T*>(p.src[v.s]) + int64_t(tok) * p.token_stride + v.head * D;
+      return v;
+    };
+    auto store_planes = [&](int r, int col, float2 v) {
+      uint32_t hi, lo;
+      split_words(v, hi, lo);
+      *reinterpret_cast<uint32_t*>(a_hi + r * kTileLd + col) = hi;
+      *reinterpret_cast<uint32_t*>(a_lo + r * kTileLd + col) = lo;
+    };
+#pragma unroll 1
+    for (uint32_t base = 0; base < n; base += 16) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const Entry v = entry(base + wg + 8 * i);
+        const float inv = 1.f / (v.nrm + 1e-10f);
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        if (v.x) load4(v.x + 4 * lane, x);
+        store_planes(wg + 8 * i, 4 * lane, make_float2(x[0] * inv, x[1] * inv));
+        store_planes(wg + 8 * i, 4 * lane + 2, make_float2(x[2] * inv, x[3] * inv));
+      }
+      group_sync(group);
+      const Entry to[2] = {entry(base + g), entry(base + g + 8)};
+      float acc[2][4];
+      chain(0, acc);
+      uint32_t off[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float* sb = reinterpret_cast<const float*>(smem + S::kBnd) + 16 * to[k].s;
+          off[i][2 * k] = 4 * bucketize15(acc[i][2 * k], sb);
+          off[i][2 * k + 1] = 4 * bucketize15(acc[i][2 * k + 1], sb);
+          uint32_t w = code_byte(off[i][2 * k], off[i][2 * k + 1]) << (8 * t);
+          w |= __shfl_xor_sync(0xffffffffu, w, 1);
+          w |= __shfl_xor_sync(0xffffffffu, w, 2);
+          if (t == 0 && to[k].slot >= 0)
+            store_code_word(p.code[to[k].s] + to[k].slot * p.code_row_stride +
+                                int64_t(to[k].head) * p.code_head_stride + 8 * wg + 4 * i, w);
+        }
+      group_sync(group);
+      if constexpr (QJL) {
+        const unsigned char* cent = smem + S::kCent;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const uint32_t e = *reinterpret_cast<const uint32_t*>(cent + off[i][2 * k]);
+            const uint32_t o = *reinterpret_cast<const uint32_t*>(cent + off[i][2 * k + 1]);
+            const int at = (g + 8 * k) * kTileLd + 16 * wg + 8 * i + 2 * t;
+            *reinterpret_cast<uint32_t*>(a_hi + at) = prmt(e, o, 0x5410);
+            *reinterpret_cast<uint32_t*>(a_lo + at) = prmt(e, o, 0x7632);
+          }
+        group_sync(group);
+        chain(1, acc);
+        group_sync(group);
+        float ss[2] = {0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int col = 16 * wg + 8 * i + 2 * t;
+            const float2 f = to[k].x ? load_pair(to[k].x + col) : make_float2(0.f, 0.f);
+            const float2 r = make_float2(fmaf(-acc[i][2 * k], to[k].nrm, f.x),
+                                         fmaf(-acc[i][2 * k + 1], to[k].nrm, f.y));
+            ss[k] = fmaf(r.x, r.x, fmaf(r.y, r.y, ss[k]));
+            store_planes(g + 8 * k, col, r);
+          }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], 1);
+          ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], 2);
+          if (t == 0) gpart[16 * wg + g + 8 * k] = ss[k];
+        }
+        group_sync(group);
+        chain(2, acc);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint32_t b = 0u;
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            b |= ((acc[i][2 * k] >= 0.f ? 1u : 0u) | (acc[i][2 * k + 1] >= 0.f ? 2u : 0u)) << (8 * i + 2 * t);
+          b |= __shfl_xor_sync(0xffffffffu, b, 1);
+          b |= __shfl_xor_sync(0xffffffffu, b, 2);
+          if (t == 0 && to[k].slot >= 0 && to[k].s == 0) {
+            *reinterpret_cast<uint16_t*>(p.sign + to[k].slot * p.sign_row_stride + to[k].head * (D / 8) +
+                                         2 * wg) = uint16_t(b);
+            if (wg == 0) {
+              float sum = 0.f;
+#pragma unroll
+              for (int w = 0; w < 8; ++w) sum += gpart[16 * w + g + 8 * k];
+              *reinterpret_cast<float*>(p.gam + to[k].slot * p.gam_row_stride + to[k].head * 4) = sqrtf(sum);
+            }
+          }
+        }
+        group_sync(group);
+      }
+    }
+  };
+
 #pragma unroll 1
   for (; item < n_items; item += stride) {
     const int s = item >= n_tiles;
@@ -299,27 +510,70 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
     const int64_t slot_now = slot;
     const int head_now = head;
 
-    // ---- |x| over both halves, x_hat as hi / lo' planes --------------------------------------------
-    float ss0 = 0.f, ss1 = 0.f;
+    // ---- |x| over both halves, in the order of the 16-row kernel that was made for such a call ------
+    if (p.sum_by_quads) {
+      // compress_kernel: four sums t over the k-steps 0 .. 7, columns 2t, 2t+1, 2t+8, 2t+9 of each
+      float q[4] = {0.f, 0.f, 0.f, 0.f};
+      auto add = [&]() {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float2 f = f2_unpack(raw.pair(i));
-      ss0 = fmaf(f.x, f.x, ss0);
-      ss1 = fmaf(f.y, f.y, ss1);
+        for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const float2 a = raw.once(8 * ks + t), b = raw.once(8 * ks + 4 + t);
+            q[t] = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(b.x, b.x, fmaf(b.y, b.y, q[t]))));
+          }
+      };
+      if (half == 0) {
+        add();
+#pragma unroll
+        for (int t = 0; t < 4; ++t) xch[128 * t] = q[t];
+      }
+      group_sync(group);
+      if (half == 1) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q[t] = xch[128 * t];
+        add();
+        part[0] = (q[0] + q[1]) + (q[2] + q[3]);
+      }
+    } else {
+      // compress_coop_kernel: 32 sums of four, then halving
+      float q[16];
+#pragma unroll
+      for (int l = 0; l < 16; ++l) {
+        const float2 a = raw.once(2 * l), b = raw.once(2 * l + 1);
+        q[l] = fmaf(b.y, b.y, fmaf(b.x, b.x, fmaf(a.y, a.y, a.x * a.x)));
+      }
+      if (half == 1) {
+#pragma unroll
+        for (int l = 0; l < 16; ++l) xch[128 * l] = q[l];
+      }
+      group_sync(group);
+      if (half == 0) {
+#pragma unroll
+        for (int l = 0; l < 16; ++l) q[l] += xch[128 * l];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+          for (int l = 0; l < o; ++l) q[l] += q[l + o];
+        part[0] = q[0];
+      }
     }
-    part[128 * half] = ss0 + ss1;
     group_sync(group);
-    const float nrm = sqrtf(part[0] + part[128]);
+    // ---- x_hat as hi / lo' planes ----------------------------------------------------------------
+    const float nrm = sqrtf(part[0]);
     // one reciprocal per vector instead of a division per coordinate: x_hat may differ from
     // x / (n + 1e-10) in the last bit, far inside the rounding of the contraction
     const float inv = 1.f / (nrm + 1e-10f);
     {
       const uint64_t sc = f2_pack(inv, inv), sc_lo = f2_pack(inv * kLoScale, inv * kLoScale);
-      uint32_t hi[32], lo[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) split_pair(raw.pair(i), sc, sc_lo, hi[i], lo[i]);
-      tmem_st32_async(a_mine, hi);
-      tmem_st32_async(a_mine + 64, lo);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) split_pair(raw.pair(16 * c + i), sc, sc_lo, hi[i], lo[i]);
+        tmem_st16_async(a_mine + 16 * c, hi);
+        tmem_st16_async(a_mine + 64 + 16 * c, lo);
+      }
     }
     if (!two_stage) fetch(item + stride);  // under the product and the rest of this item
     product(0);
@@ -328,6 +582,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
     // ---- codes --------------------------------------------------------------------------------------
     const float b3 = reinterpret_cast<const float*>(sb)[3], b7 = reinterpret_cast<const float*>(sb)[7],
                 b11 = reinterpret_cast<const float*>(sb)[11];
+    float least = 1.f;
     uint8_t* dst = p.code[s] + slot_now * p.code_row_stride + int64_t(head_now) * p.code_head_stride +
                    32 * half;
     uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
@@ -338,11 +593,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
       tc_wait_ld(y);
       uint32_t off[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) off[i] = bucket_offset(__uint_as_float(y[i]), sb, b3, b7, b11);
-      // byte = even coordinate << 4 | odd coordinate; off = 4 * index
+      for (int i = 0; i < 16; ++i) off[i] = bucket_offset(__uint_as_float(y[i]), sb, b3, b7, b11, least);
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        w[2 * c + (i >> 2)] |= ((off[2 * i] << 2) | (off[2 * i + 1] >> 2)) << (8 * (i & 3));
+        w[2 * c + (i >> 2)] |= code_byte(off[2 * i], off[2 * i + 1]) << (8 * (i & 3));
       if constexpr (QJL) {
         if (two_stage) {  // the centroids are the next product's A (the last one is done with it)
           uint32_t a[8], b[8];
@@ -358,16 +612,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
         }
       }
     }
+    // (a zero vector's coordinates are zero in any arithmetic)
+    note(least <= kNearBoundary && nrm > 0.f && slot_now >= 0, s, nrm);
     if (slot_now >= 0) {
       if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
         reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
         reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-      } else if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) reinterpret_cast<uint32_t*>(dst)[i] = w[i];
       } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) reinterpret_cast<uint16_t*>(dst)[i] = uint16_t(w[i >> 1] >> (16 * (i & 1)));
+        for (int i = 0; i < 8; ++i) store_code_word(dst + 4 * i, w[i]);
       }
     }
     if (half == 0 && slot_now >= 0)
@@ -409,18 +662,24 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
               dead ? __int_as_float(0x7fc00000) : sqrtf(part[256] + part[384]);
         uint32_t* sign = reinterpret_cast<uint32_t*>(p.sign + slot_now * p.sign_row_stride +
                                                      head_now * (D / 8) + 8 * half);
+        least = 1.f;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t y[32], w = 0u;
           tmem_ld32_async(d_mine + 32 * c, y);
           tc_wait_ld(y);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) w |= __uint_as_float(y[i]) >= 0.f ? 1u << i : 0u;
+          for (int i = 0; i < 32; ++i) {
+            w |= __uint_as_float(y[i]) >= 0.f ? 1u << i : 0u;
+            least = fminf(least, fabsf(__uint_as_float(y[i])));
+          }
           if (slot_now >= 0) sign[c] = w;
         }
+        note(least <= kNearZero && nrm > 0.f && slot_now >= 0, s, nrm);
       }
     }
   }
+  work_off();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -428,7 +687,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) compress_tile_kernel(Compress
 }
 
 template <int DT, bool QJL>
-static int launch_compress_tile(const CompressArgs& a, int64_t n_vec, int sm_count, cudaStream_t stream) {
+static int launch_compress_tile(CompressArgs a, int64_t n_vec, bool sum_by_quads, int sm_count,
+                                cudaStream_t stream) {
+  a.sum_by_quads = sum_by_quads;
   using S = TileSmem<QJL>;
   auto kern = compress_tile_kernel<DT, QJL>;
   static thread_local int configured_device = -1;

@@ -23,8 +23,8 @@ def in_calls_of(size, x, call):
     return [torch.cat(t) for t in zip(*(call(x[i:i + size]) for i in range(0, len(x), size)))]
 
 
-# few | 16-vector tiles
-SIZES = [(128, 1184, 2300), (64, 1184, 16000)]
+# few | 16-vector tiles | 128-vector tiles
+SIZES = [(128, 1184, 2300), (128, 4700, 16300), (64, 1184, 16000)]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])

@@ -14,7 +14,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("n", [2369, 2432, 2433, 19071, 37890])
+@pytest.mark.parametrize("n", [4737, 4864, 4865, 19071, 37890])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_compress(consts, dtype, n, offset):
     rot, b4 = consts["rotation_128_0"], consts["boundaries_128_4"]
@@ -28,7 +28,7 @@ def test_compress(consts, dtype, n, offset):
     check_norms(norms, ref_n)
 
 
-@pytest.mark.parametrize("heads,tokens", [(1, 2500), (3, 803), (8, 300), (8, 2500)])
+@pytest.mark.parametrize("heads,tokens", [(1, 5000), (3, 1603), (8, 600), (8, 2500)])
 @pytest.mark.parametrize("two_stage", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_append(consts, heads, tokens, two_stage, dtype):
@@ -73,3 +73,19 @@ def test_append(consts, heads, tokens, two_stage, dtype):
         check_gamma(q[:, heads * 16:].contiguous().view(torch.float32), gamma, k, codes, idx, norms,
                     rot, c3)
         check_signs(q[:, :heads * 16].reshape(-1, heads, 16), signs, k, codes, idx, norms, rot, c3, S)
+
+
+def test_more_rechecks_than_a_group_notes(consts):
+    """Every vector has a coordinate next to a boundary: a call of 262 144 of them overflows the groups' lists,
+    and each rechecks all of its vectors.  The same bytes as from a call whose lists hold them."""
+    rot, b4 = consts["rotation_128_0"].to(DEV), consts["boundaries_128_4"].to(DEV)
+    x = torch.randn(131072, 128, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV).bfloat16()
+    y = x.double() / x.double().norm(dim=-1, keepdim=True) @ rot.double().T
+    close = ((y.unsqueeze(-1) - b4.double()).abs().amin(dim=(1, 2)) < 0.8 * 2.0 ** -22).nonzero().flatten()
+    assert close.numel() >= 64
+    x = x[close[:64]].repeat(4096, 1).unsqueeze(1).contiguous()
+    packed, norms = fq.tq4_compress(x, rot, b4)
+    few = 16384  # the smallest call that sums the squares in the same order
+    want_p, want_n = fq.tq4_compress(x[:few].contiguous(), rot, b4)
+    assert torch.equal(packed[:few], want_p) and torch.equal(norms[:few], want_n)
+    assert torch.equal(packed.view(4096, -1), packed[:64].view(1, -1).expand(4096, -1))
