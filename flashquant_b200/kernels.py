@@ -847,18 +847,20 @@ def fused_tq_attention(
 
 
 def _buffer_view_capacity(codes: torch.Tensor, norms: torch.Tensor) -> int:
-    """Tokens per (batch, head) row of the buffers that ``codes`` / ``norms`` are views of."""
+    """Tokens per (batch, head) row of the buffers that ``codes`` / ``norms`` are views of (``n``
+    where there is one row).  Strides of dimensions of size one say nothing and are not looked at."""
     b, h, n, half = codes.shape
     if n == 0:
         return 0
-    if codes.stride(3) != 1 or codes.stride(2) != half or codes.stride(1) % half:
-        raise ValueError("packed codes must be a [:, :, :n] view of a contiguous buffer")
-    cap = codes.stride(1) // half
-    if b > 1 and codes.stride(0) != h * codes.stride(1):
-        raise ValueError("packed codes must be a [:, :, :n] view of a contiguous buffer")
-    nn = norms.reshape(b, h, n) if norms.dim() == 4 else norms
-    if nn.stride(2) != 1 or nn.stride(1) != cap or (b > 1 and nn.stride(0) != h * cap):
-        raise ValueError("norms must be a view of a buffer with the capacity of the codes")
+    rows = 1 if h > 1 else 0  # the dimension whose stride is the capacity
+    cap = n if b * h == 1 else codes.stride(rows) // half
+    norms = norms if norms.dim() == 4 else norms.unsqueeze(3)
+    for t, unit, what in ((codes, half, "packed codes must be a [:, :, :n] view of a contiguous buffer"),
+                          (norms, 1, "norms must be a view of a buffer with the capacity of the codes")):
+        strides = (h * cap * unit, cap * unit, unit, 1)
+        if tuple(t.shape) != (b, h, n, unit) or cap < n or any(
+                size > 1 and have != want for size, have, want in zip(t.shape, t.stride(), strides)):
+            raise ValueError(what)
     return cap
 
 

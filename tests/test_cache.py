@@ -24,6 +24,32 @@ def T(a):
     return torch.from_numpy(np.ascontiguousarray(a))
 
 
+def test_capacity_of_buffer_views():
+    """Part-filled buffers with one KV head or one batch row too, and rows whose size-one dimensions
+    carry any stride; views of something else are refused."""
+    cap = fq.kernels._buffer_view_capacity
+
+    def buffers(b, h, c):
+        return torch.zeros(b, h, c, 64, dtype=torch.uint8), torch.zeros(b, h, c, 1)
+
+    for b, h in ((1, 1), (3, 1), (1, 4), (3, 4)):
+        codes, norms = buffers(b, h, 22)
+        for n in (1, 17, 22):
+            want = n if b * h == 1 else 22
+            views = codes[:, :, :n], norms[:, :, :n]
+            assert cap(*views) == want
+            assert cap(views[0], views[1].squeeze(3)) == want
+    # (1, 1, N, 64) out of (N, 1, 64) rows: contiguous, with stride 64 in the head dimension
+    rows = torch.zeros(9, 1, 64, dtype=torch.uint8), torch.zeros(9, 1, 1)
+    assert cap(*(t.transpose(0, 1).unsqueeze(0) for t in rows)) == 9
+    codes, norms = buffers(2, 4, 22)
+    for bad in ((codes[:, :, :5], norms[:, :, :5].contiguous()), (codes[:, :, ::2], norms[:, :, ::2]),
+                (codes[:, :1, :5].expand(2, 4, 5, 64), norms[:, :, :5]),
+                (codes[:, :, :5], norms[:, :, :6])):
+        with pytest.raises(ValueError):
+            cap(*bad)
+
+
 class MockDynamicLayer:
     def __init__(self):
         self.keys = None
