@@ -368,18 +368,20 @@ PyObject* compress(PyObject*, Args a, Py_ssize_t n) {
 }
 
 // Tokens between the (batch, head) rows of the buffers that codes and norms are [:, :, :n] views
-// of; 0 if they are not.
+// of (n where there is one row); 0 if they are not.  Strides of dimensions of size one say nothing.
 int64_t view_capacity(const Tensor& codes, const Tensor& norms) {
   const int64_t b = codes.size(0), h = codes.size(1), n = codes.size(2), half = codes.size(3);
-  if (n == 0 || norms.dim() != 4 || norms.size(0) != b || norms.size(1) != h ||
+  if (n == 0 || half == 0 || norms.dim() != 4 || norms.size(0) != b || norms.size(1) != h ||
       norms.size(2) != n || norms.size(3) != 1)
     return 0;
-  if (codes.stride(3) != 1 || codes.stride(2) != half || codes.stride(1) % half) return 0;
-  const int64_t cap = codes.stride(1) / half;
-  if (b > 1 && codes.stride(0) != h * codes.stride(1)) return 0;
-  if (norms.stride(2) != 1 || norms.stride(1) != cap || (b > 1 && norms.stride(0) != h * cap))
-    return 0;
-  return cap;
+  const int64_t cap = b * h == 1 ? n : codes.stride(h > 1 ? 1 : 0) / half;
+  const auto laid_out = [&](const Tensor& t, int64_t unit) {
+    const int64_t want[4] = {h * cap * unit, cap * unit, unit, 1};
+    for (int i = 0; i < 4; ++i)
+      if (t.size(i) > 1 && t.stride(i) != want[i]) return false;
+    return true;
+  };
+  return cap >= n && laid_out(codes, half) && laid_out(norms, 1) ? cap : 0;
 }
 
 // (q, k_packed, k_norms, v_packed, v_norms, centroids_k, centroids_v, rotation_k, rotation_v,

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("hq,hkv", [(6, 2), (8, 2), (16, 2), (32, 8), (64, 64)])
+@pytest.mark.parametrize("hq,hkv", [(1, 1), (6, 2), (8, 2), (16, 2), (32, 8), (64, 64)])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 255, 273, 4099])
 @pytest.mark.parametrize("k_bits,dtype", [(3, torch.float16), (4, torch.bfloat16)])
 def test_one_token(consts, hq, hkv, n, k_bits, dtype):
@@ -38,6 +38,8 @@ def test_one_token(consts, hq, hkv, n, k_bits, dtype):
         norms[:, :, :n] = nm.view(b, hkv, n, 1)
         bufs += [codes.to(DEV)[:, :, :n], norms.to(DEV)[:, :, :n]]
     got = fq.fused_tq_attention_kv(q.to(DEV), *bufs, ck, cv, rot_k, rot_v)
+    direct = fq.fused_tq_attention_kv(q.to(DEV), *bufs, *(t.to(DEV) for t in (ck, cv, rot_k, rot_v)))
+    assert torch.equal(got, direct)
     # the rotated query is rounded to its type, everything else in 64 bits
     q_rot = (q.double() @ rot_k.double().T).to(dtype).double().view(b, hkv, hq // hkv, d)
     s = torch.softmax(q_rot @ deq[0].transpose(-1, -2) / math.sqrt(d), dim=-1)

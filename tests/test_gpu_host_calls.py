@@ -56,3 +56,28 @@ def test_strided_tokens_and_streams(consts):
     assert K.decode_workspace(torch.device(DEV), 1, 8, 8, 128, 0).data_ptr() == first.data_ptr()
     with pytest.raises(ValueError):
         fq.tq4_compress_append(k, v, a[..., :-1].contiguous(), slots, rot, bk, bv)
+
+
+@pytest.mark.parametrize("n", [1, 40])
+@pytest.mark.parametrize("b", [1, 3])
+def test_attention_over_one_kv_head(consts, b, n):
+    """One KV head: rows as the compressor returns them, turned so that the head dimension has a
+    stride of its own, and part-filled buffers; constants on the device and on the CPU."""
+    host = [consts[x].contiguous() for x in ("boundaries_128_4", "centroids_128_4", "rotation_128_0")]
+    bnd, c, rot = (t.to(DEV) for t in host)
+    q = torch.randn(b, 4, 1, 128, device=DEV).to(torch.float16)
+    kv = []
+    for _ in range(2):
+        x = torch.randn(b * n, 1, 128, device=DEV).to(torch.float16)
+        kv += [t.view(b, n, 1, -1).transpose(1, 2) for t in fq.tq4_compress(x, rot, bnd)]
+    want = fq.fused_tq_attention(q, *(t.contiguous() for t in kv), c, c, rot)
+    views = []
+    for t in kv:
+        buf = torch.zeros(b, 1, n + 7, t.shape[3], dtype=t.dtype, device=DEV)
+        buf[:, :, :n] = t
+        views.append(buf[:, :, :n])
+    for cc, rr in ((c, rot), (host[1], host[2])):
+        assert torch.equal(fq.fused_tq_attention(q, *kv, cc, cc, rr), want)
+        assert torch.equal(fq.fused_tq_attention(q, *views, cc, cc, rr), want)
+        assert torch.equal(fq.fused_tq_attention_kv(q, *views, cc, cc, rr, rr), want)
+        assert torch.equal(fq.fused_tq_attention_kv(q, *kv, cc, cc, rr, rr), want)
