@@ -611,17 +611,21 @@ static int attention_prep(PrefillArgs& a, unsigned char* ws, const float* rot_q,
 
 constexpr int kPfMaxSplits = 64;  // slices of the keys for a single query token
 
+// Head (status word, scale record) and the rotations' planes: all that prefill_pair_kernel needs.
+constexpr size_t kPairWorkspaceBytes = 256 + 2 * kPlaneBytes;
+
 struct PrefillWorkspace {
   size_t q_rot_off, o_rot_off, part_off, total;
 };
-// single_token: room for the partial rows of kPfMaxSplits slices behind the rotated output
+// One query token: behind those the rotated query and output of the 128-row tile kernel and the partial
+// rows of kPfMaxSplits slices.
 static PrefillWorkspace prefill_workspace(int64_t rows, int d, bool single_token) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   PrefillWorkspace w;
-  w.q_rot_off = 256 + 2 * kPlaneBytes;
+  w.q_rot_off = kPairWorkspaceBytes;
   w.o_rot_off = up(w.q_rot_off + size_t(rows) * d * 2);
   w.part_off = up(w.o_rot_off + size_t(rows) * d * 4);
-  w.total = single_token ? up(w.part_off + size_t(kPfMaxSplits) * rows * (d + 4) * 4) : w.part_off;
+  w.total = single_token ? up(w.part_off + size_t(kPfMaxSplits) * rows * (d + 4) * 4) : kPairWorkspaceBytes;
   return w;
 }
 
@@ -790,7 +794,7 @@ extern "C" int fq_fused_tq_attention_kv(const void* q, fq_dtype dtype, const uin
 extern "C" size_t fq_paged_tq4_prefill_workspace_bytes(int total_q_tokens, int num_q_heads,
                                                        int head_dim) {
   if (total_q_tokens < 0 || num_q_heads < 0 || head_dim < 0) return 0;
-  return prefill_workspace(int64_t(total_q_tokens) * num_q_heads, head_dim, false).total;
+  return kPairWorkspaceBytes;
 }
 
 extern "C" int fq_paged_tq4_prefill(const void* q, fq_dtype dtype, const uint8_t* kv_cache,
@@ -826,10 +830,9 @@ extern "C" int fq_paged_tq4_prefill(const void* q, fq_dtype dtype, const uint8_t
              "paged prefill: more than 65535 sequences or query heads");
   FQ_REQUIRE(aligned(q, 16) && aligned(out, 16) && aligned(kv_cache, 16) && aligned(rotation, 16),
              FQ_ERR_ALIGNMENT, "paged prefill: q, out, the cache and the rotation must be 16-byte aligned");
-  const int64_t rows = int64_t(total_q_tokens) * num_q_heads;
-  const PrefillWorkspace w = prefill_workspace(rows, head_dim, false);
-  FQ_REQUIRE(workspace && aligned(workspace, 256) && workspace_bytes >= w.total, FQ_ERR_WORKSPACE,
-             "paged prefill: workspace of %zu bytes needed (256-byte aligned)", w.total);
+  FQ_REQUIRE(workspace && aligned(workspace, 256) && workspace_bytes >= kPairWorkspaceBytes,
+             FQ_ERR_WORKSPACE, "paged prefill: workspace of %zu bytes needed (256-byte aligned)",
+             kPairWorkspaceBytes);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   PrefillArgs a{};

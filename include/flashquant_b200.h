@@ -463,7 +463,8 @@ int fq_split_k_merge(const float* partials, int n_groups, const float* rotation,
  *   k_packed, v_packed  (batch, num_kv_heads, n_kv, head_dim/2) bytes, 16-byte aligned
  *   k_norms, v_norms    (batch, num_kv_heads, n_kv) fp32
  *   workspace           caller-owned, 256-byte aligned, fq_fused_tq_attention_workspace_bytes(...)
- *                       bytes (rotated fp16 query and fp32 rotated output); first word = status
+ *                       bytes (the rotations as MMA operands; for one query token partial rows);
+ *                       first word = status, zero it before the first call
  * head_dim 128; with is_causal, n_q must equal n_kv (or be 1).
  */
 size_t fq_fused_tq_attention_workspace_bytes(int batch, int num_q_heads, int n_q, int head_dim);
@@ -517,8 +518,8 @@ int fq_fused_tq_attention_kv(const void* q, fq_dtype dtype, const uint8_t* k_pac
  *                   inside [0, total_q_tokens), sets FQ_DEV_BAD_LENGTH and is cut / skipped
  *   rounding        q Pi^T and the attention rows are rounded to the activation type before
  *                   the products with K and Pi, as the reference's two matmul + cast steps do
- *   workspace       256-byte aligned, fq_paged_tq4_prefill_workspace_bytes(...) bytes; word 0
- *                   is the status word (zero it before the first call)
+ *   workspace       256-byte aligned, fq_paged_tq4_prefill_workspace_bytes(...) bytes (128 KiB
+ *                   whatever the chunks); word 0 is the status word (zero it before the first call)
  * head_dim 128 and a multiple of 4 KV heads (16-byte gathers from the token rows) only.
  */
 size_t fq_paged_tq4_prefill_workspace_bytes(int total_q_tokens, int num_q_heads, int head_dim);

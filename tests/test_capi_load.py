@@ -71,8 +71,12 @@ def test_host_step_layout_and_new_entry_points_need_no_gpu(lib_path):
     assert lib.fq_decode_step_offsets(32, 32, 8, 128, 256, 1, None) == -1
     assert lib.fq_decode_step_offsets(-1, 32, 8, 128, 256, 1, off) == -1
     # paged prefill: sizes, and refusals that precede every launch
+    # (status word, scale record and the fp16 planes of the rotation: nothing per query row)
     need = lib.fq_paged_tq4_prefill_workspace_bytes(1000, 32, 128)
-    assert need >= 256 + 1000 * 32 * 128 * (2 + 4)
+    assert 256 + 2 * 128 * 128 * 2 <= need <= 1 << 18
+    assert lib.fq_paged_tq4_prefill_workspace_bytes(100000, 64, 128) == need
+    assert lib.fq_fused_tq_attention_workspace_bytes(4, 32, 8192, 128) == need
+    assert lib.fq_fused_tq_attention_workspace_bytes(4, 32, 1, 128) >= need + 64 * 4 * 32 * 132 * 4
     assert lib.fq_paged_tq4_prefill_workspace_bytes(-1, 32, 128) == 0
     args = [None, 2, None, None, 4, None, None, None, 8, None, 16, None, 2, 100, 50, 32, 8, 128, 16,
             64, 0.1, None, None, 0, None]
