@@ -114,7 +114,13 @@ Tensor workspace(int dev, int use, size_t bytes) {
   all[key] = t;
   return t;
 }
-enum { kDecode = 0, kAttention = 1, kPrefill = 2, kScratch = 3 };
+enum { kDecode = 0, kAttention = 1 };
+
+// Bytes for one call: what a call writes and reads back within itself is not shared with another one.
+Tensor call_bytes(int dev, size_t bytes, bool zero) {
+  const auto options = at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte);
+  return zero ? at::zeros({int64_t(bytes)}, options) : at::empty({int64_t(bytes)}, options);
+}
 
 PyObject* py_workspace(PyObject*, Args a, Py_ssize_t n) {
   int64_t dev, use;
@@ -306,8 +312,9 @@ PyObject* paged_decode_multi(PyObject*, Args a, Py_ssize_t n) {
                                      seqs, n_q, p.hq, p.hkv, p.d, p.splits),
                                  fq_paged_decode_workspace_bytes(seqs * n_q, p.hq, p.hkv, p.d,
                                                                  p.splits)));
-  Tensor scratch = workspace(
-      dev, kScratch, fq_split_k_paged_decode_multi_scratch_bytes(seqs, n_q, max_blocks));
+  Tensor scratch = call_bytes(
+      dev, std::max<size_t>(fq_split_k_paged_decode_multi_scratch_bytes(seqs, n_q, max_blocks), 16),
+      false);
   return done(fq_split_k_paged_decode_multi(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<int32_t>(*p.table),
                   p.table->stride(0), max_blocks, data<int32_t>(*p.lens), data(*p.ck),
@@ -332,7 +339,7 @@ PyObject* paged_prefill(PyObject*, Args a, Py_ssize_t n) {
       !decode_out(a[11], *p.q, dev, out) || cu->numel() != p.lens->numel() + 1)
     return none();
   const int total = int(p.q->size(0));
-  Tensor ws = workspace(dev, kPrefill, fq_paged_tq4_prefill_workspace_bytes(total, p.hq, p.d));
+  Tensor ws = call_bytes(dev, fq_paged_tq4_prefill_workspace_bytes(total, p.hq, p.d), true);
   return done(fq_paged_tq4_prefill(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<int32_t>(*p.table),
                   p.table->stride(0), data<int32_t>(*p.lens), data<int32_t>(*cu), data(*p.ck),

@@ -395,7 +395,7 @@ def tq4_compress_append_qjl(key, value, kv_cache, kq_cache, slot_mapping, rotati
 # --------------------------------------------------------------------------------------
 
 # uses of the cached workspaces (one per device, stream and use)
-_DECODE, _ATTENTION, _PREFILL = 0, 1, 2
+_DECODE, _ATTENTION = 0, 1
 
 
 def _workspace(device, use: int, need: int) -> torch.Tensor:
@@ -624,7 +624,7 @@ def paged_tq4_prefill(q, kv_cache, block_table, seq_lens, cu_seqlens_q, max_q_le
     lib = N.load()
     need = lib.fq_paged_tq4_prefill_workspace_bytes(total, hq, d)
     if workspace is None:
-        workspace = _workspace(dev, _PREFILL, need)
+        workspace = torch.zeros(need, dtype=torch.uint8, device=dev)
     N.check(lib.fq_paged_tq4_prefill(
         N.ptr(q), N.dtype_code(q.dtype), N.ptr(kv_cache), N.ptr(block_table),
         block_table.stride(0), N.ptr(seq_lens), N.ptr(cu), N.ptr(ck), ck.numel(), N.ptr(cv),

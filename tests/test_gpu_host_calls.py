@@ -81,3 +81,33 @@ def test_attention_over_one_kv_head(consts, b, n):
         assert torch.equal(fq.fused_tq_attention(q, *views, cc, cc, rr), want)
         assert torch.equal(fq.fused_tq_attention_kv(q, *views, cc, cc, rr, rr), want)
         assert torch.equal(fq.fused_tq_attention_kv(q, *kv, cc, cc, rr, rr), want)
+
+
+def test_recorded_multi_token_call_after_a_larger_one(consts):
+    """A call recorded in a CUDA graph on a stream that had run one before, then a call with a much wider
+    block table on that stream: the replay writes nothing into memory that has been handed on."""
+    w = W.decode_workload(seq_lens=[40, 700], num_q_heads=32, num_kv_heads=8, cfg=62)
+    k, v = (t.to(DEV) for t in W.make_kv(w.total_tokens, 8, 128, 62))
+    rot, bk, bv, ck, cv = (consts[n].contiguous().to(DEV) for n in (
+        "rotation_128_0", "boundaries_128_3", "boundaries_128_4", "centroids_128_3", "centroids_128_4"))
+    cache = torch.zeros(w.num_blocks, 16, 8 * 136, dtype=torch.uint8, device=DEV)
+    fq.tq4_compress_append(k, v, cache, w.slot_mapping.to(DEV), rot, bk, bv)
+    q = w.q.to(DEV)[:, None].repeat(1, 3, 1, 1)  # (three tokens: rows in scratch memory)
+    table, lens = w.block_table.to(DEV), w.seq_lens.to(DEV)
+    wide = torch.zeros(2, 100000, dtype=torch.int32, device=DEV)
+    wide[:, :table.shape[1]] = table
+    call = lambda t: fq.split_k_paged_decode_multi(q, cache, t, lens, ck, cv, rot, 8, 128, 16)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        want = call(table)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = call(table)
+        assert torch.equal(call(wide), want)
+        others = [torch.zeros(1 << 20, dtype=torch.uint8, device=DEV) for _ in range(8)]
+        graph.replay()
+        stream.synchronize()
+        assert torch.equal(out, want)
+        assert not any(bool(t.any()) for t in others)
+    graph.reset()
