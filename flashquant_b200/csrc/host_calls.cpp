@@ -13,10 +13,12 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "flashquant_b200.h"
 
@@ -92,27 +94,24 @@ T* data(const Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 
 // ------------------------------------------------------------------------------------
 // Workspaces: one per (device, stream, use), zero at first use, grown on demand.  Calls on
-// different streams may overlap on the GPU and must not share counters or partial rows.  At most
-// kMaxWorkspaces are kept (a program that goes through more streams than that starts over: the
-// allocator gives a dropped block to later work of the same stream only).
+// different streams may overlap on the GPU and must not share counters or partial rows.  None is given
+// back: a call recorded in a CUDA graph keeps the address, so a workspace that was outgrown stays too
+// (each is at least twice its predecessor, all of them together less than twice the last).
 // ------------------------------------------------------------------------------------
-constexpr size_t kMaxWorkspaces = 64;
 std::mutex g_ws_mutex;
-std::map<std::tuple<int, const void*, int>, Tensor>& workspaces() {
-  static auto* m = new std::map<std::tuple<int, const void*, int>, Tensor>();
+std::map<std::tuple<int, const void*, int>, std::vector<Tensor>>& workspaces() {
+  static auto* m = new std::map<std::tuple<int, const void*, int>, std::vector<Tensor>>();
   return *m;  // never destroyed: the CUDA context may be gone at exit
 }
 Tensor workspace(int dev, int use, size_t bytes) {
   const auto key = std::make_tuple(dev, static_cast<const void*>(stream_of(dev)), use);
   std::lock_guard<std::mutex> lock(g_ws_mutex);
-  auto& all = workspaces();
-  auto it = all.find(key);
-  if (it != all.end() && size_t(it->second.numel()) >= bytes) return it->second;
-  if (it == all.end() && all.size() >= kMaxWorkspaces) all.clear();
-  const size_t n = bytes < (size_t(1) << 20) ? (size_t(1) << 20) : bytes;
-  Tensor t = at::zeros({int64_t(n)}, at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte));
-  all[key] = t;
-  return t;
+  auto& kept = workspaces()[key];
+  const size_t have = kept.empty() ? size_t(1) << 19 : size_t(kept.back().numel());
+  if (kept.empty() || have < bytes)
+    kept.push_back(at::zeros({int64_t(std::max(bytes, 2 * have))},
+                             at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte)));
+  return kept.back();
 }
 enum { kDecode = 0, kAttention = 1 };
 

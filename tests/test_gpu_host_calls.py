@@ -111,3 +111,26 @@ def test_recorded_multi_token_call_after_a_larger_one(consts):
         assert torch.equal(out, want)
         assert not any(bool(t.any()) for t in others)
     graph.reset()
+
+
+def test_workspaces_stay_where_they_are():
+    """The address that a recorded call holds: neither many streams nor a larger call moves it to
+    other hands."""
+    dev = torch.device(DEV)
+    first = K.decode_workspace(dev, 1, 8, 8, 128, 0)
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(33)]
+    with torch.cuda.stream(streams[0]):
+        small = K.decode_workspace(dev, 1, 8, 8, 128, 0)
+    at, size = small.data_ptr(), small.numel()
+    del small
+    for s in streams:
+        with torch.cuda.stream(s):
+            for use in (K._DECODE, K._ATTENTION):
+                K._workspace(dev, use, 0)
+    assert K.decode_workspace(dev, 1, 8, 8, 128, 0).data_ptr() == first.data_ptr()
+    with torch.cuda.stream(streams[0]):
+        assert K.decode_workspace(dev, 1, 8, 8, 128, 0).data_ptr() == at
+        large = K._workspace(dev, K._DECODE, size + 1)
+        assert large.data_ptr() != at and large.numel() >= 2 * size
+        others = [torch.empty(1 << 20, dtype=torch.uint8, device=dev) for _ in range(16)]
+    assert not any(t.data_ptr() < at + size and at < t.data_ptr() + t.numel() for t in others)
