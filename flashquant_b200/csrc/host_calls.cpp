@@ -121,6 +121,25 @@ Tensor call_bytes(int dev, size_t bytes, bool zero) {
   return zero ? at::zeros({int64_t(bytes)}, options) : at::empty({int64_t(bytes)}, options);
 }
 
+// (device_index, use) -> the workspaces of all streams
+PyObject* py_workspaces(PyObject*, Args a, Py_ssize_t n) {
+  int64_t dev, use;
+  if (n != 2 || !as_int(a[0], dev) || !as_int(a[1], use)) {
+    PyErr_SetString(PyExc_TypeError, "workspaces(device_index, use)");
+    return nullptr;
+  }
+  PyObject* list = PyList_New(0);
+  std::lock_guard<std::mutex> lock(g_ws_mutex);
+  for (const auto& [key, kept] : workspaces())
+    if (std::get<0>(key) == dev && std::get<2>(key) == use)
+      for (const Tensor& t : kept) {
+        PyObject* o = list ? THPVariable_Wrap(t) : nullptr;
+        if (!o || PyList_Append(list, o)) Py_CLEAR(list);
+        Py_XDECREF(o);
+      }
+  return list;
+}
+
 PyObject* py_workspace(PyObject*, Args a, Py_ssize_t n) {
   int64_t dev, use;
   if (n != 3 || !as_int(a[0], dev) || !as_int(a[1], use) || !PyLong_Check(a[2])) {
@@ -499,6 +518,8 @@ PyMethodDef kMethods[] = {
     FQ_METHOD(compress_append), FQ_METHOD(compress_append_qjl), FQ_METHOD(paged_decode),
     FQ_METHOD(paged_decode_qjl), FQ_METHOD(paged_decode_multi), FQ_METHOD(paged_prefill),
     FQ_METHOD(compress), FQ_METHOD(attention), FQ_METHOD(cache_update),
+    {"workspaces", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&py_workspaces)),
+     METH_FASTCALL, nullptr},
     {"workspace", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&py_workspace)),
      METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -916,5 +916,11 @@ def fused_tq_attention_kv(
 
 
 def attention_workspace_status(device) -> int:
-    """Device status word of the current stream's attention workspace (0 = no error)."""
-    return workspace_status(_workspace(device, _ATTENTION, 0))
+    """Device status word of the device's attention workspaces, those of all streams together (0 = no
+    error).  Waits for the current stream only."""
+    device = torch.device(device)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    status = 0
+    for ws in _host().workspaces(index, _ATTENTION):
+        status |= workspace_status(ws)
+    return status

@@ -134,3 +134,15 @@ def test_workspaces_stay_where_they_are():
         assert large.data_ptr() != at and large.numel() >= 2 * size
         others = [torch.empty(1 << 20, dtype=torch.uint8, device=dev) for _ in range(16)]
     assert not any(t.data_ptr() < at + size and at < t.data_ptr() + t.numel() for t in others)
+
+
+def test_attention_status_covers_all_streams():
+    dev = torch.device(DEV)
+    K._workspace(dev, K._ATTENTION, 0)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        other = K._workspace(dev, K._ATTENTION, 0)
+    assert K.attention_workspace_status(dev) == 0
+    other[0] = 4
+    assert K.attention_workspace_status(dev) == 4 and K.attention_workspace_status("cuda") == 4
+    other[0] = 0
+    assert K.attention_workspace_status(dev) == 0
