@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import warnings
 from typing import Optional, Tuple
 
 import torch
@@ -21,13 +22,39 @@ from . import _native as N
 _host_module = None
 
 
+class _ConvertingCalls:
+    """Stands in for the extension module where only the C library has been built: takes no call, so
+    that all of them are converted and made through ctypes, and keeps the workspaces."""
+
+    def __init__(self):
+        self._kept = {}
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+    def workspace(self, index, use, need):
+        kept = self._kept.setdefault((index, torch.cuda.current_stream(index).cuda_stream, use), [])
+        have = kept[-1].numel() if kept else 1 << 19
+        if not kept or have < need:
+            kept.append(torch.zeros(max(need, 2 * have), dtype=torch.uint8, device=f"cuda:{index}"))
+        return kept[-1]
+
+    def workspaces(self, index, use):
+        return [t for key, kept in self._kept.items() if key[0] == index and key[2] == use for t in kept]
+
+
 def _host():
     """The extension module that makes a call whose arguments need no conversion (it returns None
     for the others, an int for a native status, else the result)."""
     global _host_module
     if _host_module is None:
         N.load()  # the message about a library that has not been built
-        from . import _host as m
+        try:
+            from . import _host as m
+        except ImportError as e:
+            warnings.warn(f"{e}: calls go through ctypes, about 20 us more each "
+                          "(python -m flashquant_b200.build makes the module)")
+            m = _ConvertingCalls()
         _host_module = m
     return _host_module
 

@@ -112,3 +112,18 @@ def test_pybind_module_exports_the_probed_names():
     with pytest.raises(RuntimeError):
         _C.tq4_compress(torch.randn(2, 1, 128), torch.zeros(128, 64), torch.zeros(128, 64),
                         torch.zeros(15), None)
+
+
+def test_package_without_the_extension_module(lib_path, monkeypatch):
+    """A build of the C library alone serves the package: every call is converted."""
+    import sys
+
+    import flashquant_b200
+    from flashquant_b200 import kernels as K
+    monkeypatch.setitem(sys.modules, "flashquant_b200._host", None)
+    monkeypatch.delattr(flashquant_b200, "_host", raising=False)
+    monkeypatch.setattr(K, "_host_module", None)
+    with pytest.warns(UserWarning, match="_host"):
+        host = K._host()
+    assert host.paged_decode(1, 2, 3) is None and host.compress() is None
+    assert K._host() is host and host.workspaces(0, K._ATTENTION) == []

@@ -146,3 +146,23 @@ def test_attention_status_covers_all_streams():
     assert K.attention_workspace_status(dev) == 4 and K.attention_workspace_status("cuda") == 4
     other[0] = 0
     assert K.attention_workspace_status(dev) == 0
+
+
+def test_calls_without_the_extension_module(consts, monkeypatch):
+    w = W.decode_workload(seq_lens=[40, 700], num_q_heads=32, num_kv_heads=8, cfg=63)
+    k, v = (t.to(DEV) for t in W.make_kv(w.total_tokens, 8, 128, 63))
+    rot, bk, bv, ck, cv = (consts[n].contiguous().to(DEV) for n in (
+        "rotation_128_0", "boundaries_128_3", "boundaries_128_4", "centroids_128_3", "centroids_128_4"))
+
+    def run():
+        cache = torch.zeros(w.num_blocks, 16, 8 * 136, dtype=torch.uint8, device=DEV)
+        fq.tq4_compress_append(k, v, cache, w.slot_mapping.to(DEV), rot, bk, bv)
+        return cache, fq.split_k_paged_decode(w.q.to(DEV), cache, w.block_table.to(DEV),
+                                              w.seq_lens.to(DEV), ck, cv, rot, 8, 128, 16)
+
+    want = run()
+    monkeypatch.setattr(K, "_host_module", K._ConvertingCalls())
+    assert all(torch.equal(a, b) for a, b in zip(run(), want))
+    ws = K.decode_workspace(torch.device(DEV), 2, 32, 8, 128, 0)
+    assert ws.data_ptr() == K.decode_workspace(torch.device(DEV), 2, 32, 8, 128, 0).data_ptr()
+    assert K.attention_workspace_status(DEV) == 0
