@@ -98,20 +98,48 @@ T* data(const Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 // back: a call recorded in a CUDA graph keeps the address, so a workspace that was outgrown stays too
 // (each is at least twice its predecessor, all of them together less than twice the last).
 // ------------------------------------------------------------------------------------
+struct Workspace {
+  std::vector<Tensor> kept;  // the last one is in use
+  std::mutex calls;          // held while a call that uses it is enqueued
+};
 std::mutex g_ws_mutex;
-std::map<std::tuple<int, const void*, int>, std::vector<Tensor>>& workspaces() {
-  static auto* m = new std::map<std::tuple<int, const void*, int>, std::vector<Tensor>>();
+std::map<std::tuple<int, const void*, int>, Workspace>& workspaces() {
+  static auto* m = new std::map<std::tuple<int, const void*, int>, Workspace>();
   return *m;  // never destroyed: the CUDA context may be gone at exit
 }
-Tensor workspace(int dev, int use, size_t bytes) {
+// `calls`: receives the lock of the workspace's calls
+Tensor workspace(int dev, int use, size_t bytes, std::mutex** calls = nullptr) {
   const auto key = std::make_tuple(dev, static_cast<const void*>(stream_of(dev)), use);
+  size_t have = size_t(1) << 19;
+  {
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    Workspace& w = workspaces()[key];
+    if (calls) *calls = &w.calls;
+    if (!w.kept.empty()) {
+      have = size_t(w.kept.back().numel());
+      if (have >= bytes) return w.kept.back();
+    }
+  }
+  // (not under the lock: an allocation may run Python code, which may pass the interpreter on)
+  Tensor t = at::zeros({int64_t(std::max(bytes, 2 * have))},
+                       at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte));
   std::lock_guard<std::mutex> lock(g_ws_mutex);
-  auto& kept = workspaces()[key];
-  const size_t have = kept.empty() ? size_t(1) << 19 : size_t(kept.back().numel());
-  if (kept.empty() || have < bytes)
-    kept.push_back(at::zeros({int64_t(std::max(bytes, 2 * have))},
-                             at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte)));
+  auto& kept = workspaces()[key].kept;
+  if (kept.empty() || size_t(kept.back().numel()) < size_t(t.numel())) kept.push_back(t);
   return kept.back();
+}
+// The native call without the interpreter lock (a full launch queue makes it wait), and alone among the
+// calls that use the same workspace: it may be several launches.
+struct WithoutInterpreter {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutInterpreter() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+int native(std::mutex* calls, F call) {
+  WithoutInterpreter released;
+  std::unique_lock<std::mutex> lock;
+  if (calls) lock = std::unique_lock<std::mutex>(*calls);
+  return call();
 }
 enum { kDecode = 0, kAttention = 1 };
 
@@ -128,15 +156,19 @@ PyObject* py_workspaces(PyObject*, Args a, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "workspaces(device_index, use)");
     return nullptr;
   }
+  std::vector<Tensor> found;
+  {
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    for (const auto& [key, w] : workspaces())
+      if (std::get<0>(key) == dev && std::get<2>(key) == use)
+        found.insert(found.end(), w.kept.begin(), w.kept.end());
+  }
   PyObject* list = PyList_New(0);
-  std::lock_guard<std::mutex> lock(g_ws_mutex);
-  for (const auto& [key, kept] : workspaces())
-    if (std::get<0>(key) == dev && std::get<2>(key) == use)
-      for (const Tensor& t : kept) {
-        PyObject* o = list ? THPVariable_Wrap(t) : nullptr;
-        if (!o || PyList_Append(list, o)) Py_CLEAR(list);
-        Py_XDECREF(o);
-      }
+  for (const Tensor& t : found) {
+    PyObject* o = list ? THPVariable_Wrap(t) : nullptr;
+    if (!o || PyList_Append(list, o)) Py_CLEAR(list);
+    Py_XDECREF(o);
+  }
   return list;
 }
 
@@ -194,10 +226,12 @@ PyObject* compress_append(PyObject*, Args a, Py_ssize_t n) {
   const Tensor *rot = f32(a[4], dev), *bk = f32(a[5], dev);
   const Tensor* bv = a[6] == Py_None ? bk : f32(a[6], dev);
   if (!rot || !bk || !bv || !append_args(a[0], a[1], a[2], a[3], dev, p)) return none();
-  return done(fq_tq4_compress_append(
+  return done(native(nullptr, [&] {
+    return fq_tq4_compress_append(
       p.key->data_ptr(), p.value->data_ptr(), fq_dtype(p.dt), p.n, p.h, p.d, p.stride, data(*rot),
       data(*bk), int(bk->numel()), data(*bv), int(bv->numel()), data<uint8_t>(*p.cache),
-      p.num_slots, p.slots->data_ptr(), p.slots->scalar_type() == at::kLong, stream_of(dev)));
+      p.num_slots, p.slots->data_ptr(), p.slots->scalar_type() == at::kLong, stream_of(dev));
+  }));
 }
 
 // (key, value, kv_cache, kq_cache, slot_mapping, rotation, boundaries_k, centroids_k,
@@ -215,11 +249,13 @@ PyObject* compress_append_qjl(PyObject*, Args a, Py_ssize_t n) {
       plane->size(0) * plane->size(1) != p.num_slots || s->dim() != 2 || s->size(0) != p.d ||
       s->size(1) != p.d || ck->numel() != bk->numel() + 1)
     return none();
-  return done(fq_tq4_compress_append_qjl(
+  return done(native(nullptr, [&] {
+    return fq_tq4_compress_append_qjl(
       p.key->data_ptr(), p.value->data_ptr(), fq_dtype(p.dt), p.n, p.h, p.d, p.stride, data(*rot),
       data(*bk), int(bk->numel()), data(*ck), data(*bv), int(bv->numel()), data(*s),
       data<uint8_t>(*p.cache), data<uint8_t>(*plane), p.num_slots, p.slots->data_ptr(),
-      p.slots->scalar_type() == at::kLong, stream_of(dev)));
+      p.slots->scalar_type() == at::kLong, stream_of(dev));
+  }));
 }
 
 // ------------------------------------------------------------------------------------
@@ -278,14 +314,17 @@ PyObject* paged_decode(PyObject*, Args a, Py_ssize_t n) {
   Tensor out;
   if (!decode_args(a, a[10], a[12], dev, 3, p) || !decode_out(a[11], *p.q, dev, out)) return none();
   const int seqs = int(p.q->size(0));
+  std::mutex* calls;
   Tensor ws = workspace(dev, kDecode,
-                        fq_paged_decode_workspace_bytes(seqs, p.hq, p.hkv, p.d, p.splits));
-  return done(fq_split_k_paged_decode(
+                        fq_paged_decode_workspace_bytes(seqs, p.hq, p.hkv, p.d, p.splits), &calls);
+  return done(native(calls, [&] {
+    return fq_split_k_paged_decode(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<int32_t>(*p.table),
                   p.table->stride(0), data<int32_t>(*p.lens), data(*p.ck), int(p.ck->numel()),
                   data(*p.cv), int(p.cv->numel()), data(*p.rot), seqs, p.hq, p.hkv, p.d, p.bs,
                   p.cache->size(0), p.scale, out.data_ptr(), p.splits, ws.data_ptr(),
-                  size_t(ws.numel()), stream_of(dev)),
+                  size_t(ws.numel()), stream_of(dev));
+  }),
               out);
 }
 
@@ -304,14 +343,17 @@ PyObject* paged_decode_qjl(PyObject*, Args a, Py_ssize_t n) {
       s->size(1) != p.d)
     return none();
   const int seqs = int(p.q->size(0));
+  std::mutex* calls;
   Tensor ws = workspace(dev, kDecode,
-                        fq_paged_decode_workspace_bytes(seqs, p.hq, p.hkv, p.d, p.splits));
-  return done(fq_split_k_paged_decode_qjl(
+                        fq_paged_decode_workspace_bytes(seqs, p.hq, p.hkv, p.d, p.splits), &calls);
+  return done(native(calls, [&] {
+    return fq_split_k_paged_decode_qjl(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<uint8_t>(*plane),
                   data<int32_t>(*p.table), p.table->stride(0), data<int32_t>(*p.lens), data(*p.ck),
                   int(p.ck->numel()), data(*p.cv), int(p.cv->numel()), data(*p.rot), data(*s), seqs,
                   p.hq, p.hkv, p.d, p.bs, p.cache->size(0), p.scale, out.data_ptr(), p.splits,
-                  ws.data_ptr(), size_t(ws.numel()), stream_of(dev)),
+                  ws.data_ptr(), size_t(ws.numel()), stream_of(dev));
+  }),
               out);
 }
 
@@ -325,21 +367,25 @@ PyObject* paged_decode_multi(PyObject*, Args a, Py_ssize_t n) {
   if (seqs == 0 || n_q == 0) return none();
   Tensor out = at::empty(p.q->sizes(), p.q->options());
   const int max_blocks = int(p.table->size(1));
+  std::mutex* calls;
   Tensor ws = workspace(dev, kDecode,
                         std::max(fq_split_k_paged_decode_multi_workspace_bytes(
                                      seqs, n_q, p.hq, p.hkv, p.d, p.splits),
                                  fq_paged_decode_workspace_bytes(seqs * n_q, p.hq, p.hkv, p.d,
-                                                                 p.splits)));
+                                                                 p.splits)),
+                        &calls);
   Tensor scratch = call_bytes(
       dev, std::max<size_t>(fq_split_k_paged_decode_multi_scratch_bytes(seqs, n_q, max_blocks), 16),
       false);
-  return done(fq_split_k_paged_decode_multi(
+  return done(native(calls, [&] {
+    return fq_split_k_paged_decode_multi(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<int32_t>(*p.table),
                   p.table->stride(0), max_blocks, data<int32_t>(*p.lens), data(*p.ck),
                   int(p.ck->numel()), data(*p.cv), int(p.cv->numel()), data(*p.rot), seqs, n_q,
                   p.hq, p.hkv, p.d, p.bs, p.cache->size(0), p.scale, out.data_ptr(), p.splits,
                   ws.data_ptr(), size_t(ws.numel()), scratch.data_ptr(), size_t(scratch.numel()),
-                  stream_of(dev)),
+                  stream_of(dev));
+  }),
               out);
 }
 
@@ -358,13 +404,15 @@ PyObject* paged_prefill(PyObject*, Args a, Py_ssize_t n) {
     return none();
   const int total = int(p.q->size(0));
   Tensor ws = call_bytes(dev, fq_paged_tq4_prefill_workspace_bytes(total, p.hq, p.d), true);
-  return done(fq_paged_tq4_prefill(
+  return done(native(nullptr, [&] {
+    return fq_paged_tq4_prefill(
                   p.q->data_ptr(), fq_dtype(p.dt), data<uint8_t>(*p.cache), data<int32_t>(*p.table),
                   p.table->stride(0), data<int32_t>(*p.lens), data<int32_t>(*cu), data(*p.ck),
                   int(p.ck->numel()), data(*p.cv), int(p.cv->numel()), data(*p.rot),
                   int(p.lens->numel()), total, int(max_q), p.hq, p.hkv, p.d, p.bs,
                   p.cache->size(0), p.scale, out.data_ptr(), ws.data_ptr(), size_t(ws.numel()),
-                  stream_of(dev)),
+                  stream_of(dev));
+  }),
               out);
 }
 
@@ -381,9 +429,11 @@ PyObject* compress(PyObject*, Args a, Py_ssize_t n) {
   const int64_t nt = x->size(0), h = x->size(1), d = x->size(2);
   Tensor packed = at::empty({nt, h, d / 2}, x->options().dtype(at::kByte));
   Tensor norms = at::empty({nt, h, 1}, x->options().dtype(at::kFloat));
-  const int rc = fq_tq4_compress(x->data_ptr(), fq_dtype(dtype_code(*x)), data(*even), data(*odd),
+  const int rc = native(nullptr, [&] {
+    return fq_tq4_compress(x->data_ptr(), fq_dtype(dtype_code(*x)), data(*even), data(*odd),
                                  data(*bnd), int(bnd->numel()), data<uint8_t>(packed), data(norms),
                                  nt * h, int(d), stream_of(dev));
+  });
   if (rc != FQ_OK) return done(rc);
   PyObject* t = PyTuple_New(2);
   if (!t) return nullptr;
@@ -433,13 +483,16 @@ PyObject* attention(PyObject*, Args a, Py_ssize_t n) {
   const int64_t cap = view_capacity(*kv[0], *kv[1]);
   if (cap == 0 || view_capacity(*kv[2], *kv[3]) != cap) return none();
   Tensor out = at::empty(q->sizes(), q->options());
-  Tensor ws = workspace(dev, kAttention, fq_fused_tq_attention_workspace_bytes(b, hq, nq, d));
-  return done(fq_fused_tq_attention_kv(
+  std::mutex* calls;
+  Tensor ws = workspace(dev, kAttention, fq_fused_tq_attention_workspace_bytes(b, hq, nq, d), &calls);
+  return done(native(calls, [&] {
+    return fq_fused_tq_attention_kv(
                   q->data_ptr(), fq_dtype(dtype_code(*q)), data<uint8_t>(*kv[0]), data(*kv[1]),
                   data<uint8_t>(*kv[2]), data(*kv[3]), data(*ck), int(ck->numel()), data(*cv),
                   int(cv->numel()), data(*rk), data(*rv), b, hq, hkv, nq, nkv, cap, d, scale,
                   a[10] == Py_True, out.data_ptr(), ws.data_ptr(), size_t(ws.numel()),
-                  stream_of(dev)),
+                  stream_of(dev));
+  }),
               out);
 }
 
@@ -489,13 +542,15 @@ PyObject* cache_update(PyObject*, Args a, Py_ssize_t n) {
   } else if (a[10] != Py_None) {
     return none();
   }
-  return done(fq_cache_update(
+  return done(native(nullptr, [&] {
+    return fq_cache_update(
       key->data_ptr(), val->data_ptr(), fq_dtype(dtype_code(*key)), data(*tk[0]), data(*tk[1]),
       data(*tk[4]), data(*tv[0]), data(*tv[1]), data(*tv[4]), data(*tk[2]), int(tk[2]->numel()),
       data(*tk[3]), int(tk[3]->numel()), data<uint8_t>(*buf[0]), data(*buf[1]),
       data<uint8_t>(*buf[2]), data(*buf[3]), b * h, s, buf[0]->size(2), at,
       ko ? ko->data_ptr() : nullptr, vo ? vo->data_ptr() : nullptr, out_cap, out_at, int(d),
-      ws ? ws->data_ptr() : nullptr, need, stream_of(dev)));
+      ws ? ws->data_ptr() : nullptr, need, stream_of(dev));
+  }));
 }
 
 // C++ exceptions (an allocation that fails) become Python ones

@@ -1,6 +1,9 @@
 """The direct call path (arguments the kernels take as they are) and the converting one (constants
 on the CPU, other layouts) give the same bits, and wrong arguments still raise."""
 
+import threading
+import time
+
 import pytest
 import torch
 
@@ -166,3 +169,65 @@ def test_calls_without_the_extension_module(consts, monkeypatch):
     ws = K.decode_workspace(torch.device(DEV), 2, 32, 8, 128, 0)
     assert ws.data_ptr() == K.decode_workspace(torch.device(DEV), 2, 32, 8, 128, 0).data_ptr()
     assert K.attention_workspace_status(DEV) == 0
+
+
+def test_other_threads_run_while_a_call_waits(consts):
+    """A launch queue that is full behind half a second of other work makes a call wait; the
+    interpreter lock is free meanwhile."""
+    rot, bk = (consts[n].contiguous().to(DEV) for n in ("rotation_128_0", "boundaries_128_3"))
+    k = torch.randn(4, 8, 128, device=DEV).to(torch.bfloat16)
+    cache = torch.zeros(1, 16, 8 * 136, dtype=torch.uint8, device=DEV)
+    slots = torch.arange(4, device=DEV)
+    fq.tq4_compress_append(k, k, cache, slots, rot, bk)
+    torch.cuda.synchronize()
+    seen, stop = [], threading.Event()
+
+    def watch():
+        while not stop.is_set():
+            seen.append(time.perf_counter())
+            time.sleep(0.001)
+
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    try:
+        torch.cuda._sleep(10 ** 9)  # about 0.5 s on the stream
+        longest = 0.0
+        for _ in range(4000):
+            t = time.perf_counter()
+            fq.tq4_compress_append(k, k, cache, slots, rot, bk)
+            longest = max(longest, time.perf_counter() - t)
+        torch.cuda.synchronize()
+    finally:
+        stop.set()
+        watcher.join()
+    assert longest > 0.2, f"no call waited ({longest:.3f} s): the queue was not full"
+    gap = max(b - a for a, b in zip(seen, seen[1:]))
+    assert gap < 0.1, f"no other thread ran for {gap:.3f} s"
+
+
+def test_threads_on_one_stream(consts):
+    """Single-token attention of two threads on one stream, which share a workspace: a call is several
+    launches, and nothing of another call comes in between."""
+    bnd, c, rot = (consts[n].contiguous().to(DEV) for n in ("boundaries_128_4", "centroids_128_4", "rotation_128_0"))
+    cases = []
+    for i in range(2):
+        x = torch.randn(2 * 8 * 600, 1, 128, device=DEV, generator=torch.Generator(DEV).manual_seed(i)).half()
+        p, n = fq.tq4_compress(x, rot, bnd)
+        q = torch.randn(2, 32, 1, 128, device=DEV).half()
+        args = (q, p.view(2, 8, 600, 64), n.view(2, 8, 600, 1), p.view(2, 8, 600, 64), n.view(2, 8, 600, 1), c, c, rot)
+        cases.append((args, fq.fused_tq_attention(*args)))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    wrong = []
+
+    def run(args, want):
+        with torch.cuda.stream(stream):
+            outs = [fq.fused_tq_attention(*args) for _ in range(300)]
+            wrong.extend(i for i, o in enumerate(outs) if not torch.equal(o, want))
+
+    threads = [threading.Thread(target=run, args=case) for case in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
