@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kCompressThreads, QJL ? 1 : 2) compress_kernel
             *reinterpret_cast<uint4*>(d0) = make_uint4(keep0[0], keep0[1], keep0[2], keep0[3]);
           } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(d0)[i] = keep0[i];
+            for (int i = 0; i < 4; ++i) store_code_word(d0 + 4 * i, keep0[i]);
           }
         }
         if (slot1 >= 0) {
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kCompressThreads, QJL ? 1 : 2) compress_kernel
             *reinterpret_cast<uint4*>(d1) = make_uint4(keep1[0], keep1[1], keep1[2], keep1[3]);
           } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(d1)[i] = keep1[i];
+            for (int i = 0; i < 4; ++i) store_code_word(d1 + 4 * i, keep1[i]);
           }
         }
       }
@@ -693,11 +693,11 @@ __global__ void __launch_bounds__(kCoopThreads, QJL ? 1 : 2) compress_coop_kerne
         w_hi |= __shfl_xor_sync(0xffffffffu, w_hi, 2);
         const int byte0 = 4 * (warp * NTW + i);
         if (t == 0 && slot_lo >= 0)
-          *reinterpret_cast<uint32_t*>(p.code[s] + slot_lo * p.code_row_stride +
-                                       int64_t(head_lo) * p.code_head_stride + byte0) = w_lo;
+          store_code_word(p.code[s] + slot_lo * p.code_row_stride + int64_t(head_lo) * p.code_head_stride + byte0,
+                          w_lo);
         if (t == 1 && slot_hi >= 0)
-          *reinterpret_cast<uint32_t*>(p.code[s] + slot_hi * p.code_row_stride +
-                                       int64_t(head_hi) * p.code_head_stride + byte0) = w_hi;
+          store_code_word(p.code[s] + slot_hi * p.code_row_stride + int64_t(head_hi) * p.code_head_stride + byte0,
+                          w_hi);
       }
     }
     __syncthreads();  // every warp has read x_hat: the planes may be overwritten

@@ -219,8 +219,7 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
     w |= __shfl_xor_sync(0xffffffffu, w, 2);
     w |= __shfl_xor_sync(0xffffffffu, w, 4);
     if ((lane & 7) == 0 && slot_r >= 0)
-      *reinterpret_cast<uint32_t*>(p.code[s] + slot_r * p.code_row_stride +
-                                   int64_t(head_r) * p.code_head_stride + j / 2) = w;
+      store_code_word(p.code[s] + slot_r * p.code_row_stride + int64_t(head_r) * p.code_head_stride + j / 2, w);
   } else {
     // a warp holds columns 8*warp .. 8*warp+7 of every vector, column = lane / 4
     uint32_t w = uint32_t(idx) << (8 * (lane >> 3) + ((ja & 1) ? 0 : 4));
@@ -228,8 +227,8 @@ __global__ void __launch_bounds__(kFewVecs* D, kTwoStage ? 1 : 2)
     w |= __shfl_xor_sync(0xffffffffu, w, 8);
     w |= __shfl_xor_sync(0xffffffffu, w, 16);
     if (lane < 4 && slot_sl >= 0)
-      *reinterpret_cast<uint32_t*>(p.code[s] + slot_sl * p.code_row_stride +
-                                   int64_t(head_sl) * p.code_head_stride + 4 * warp) = w;
+      store_code_word(p.code[s] + slot_sl * p.code_row_stride + int64_t(head_sl) * p.code_head_stride + 4 * warp,
+                      w);
     if constexpr (kTwoStage) {
       __syncthreads();  // x_hat has been read
       xs[sl][ja] = s_cent[idx];

@@ -326,3 +326,37 @@ def test_two_bit_packing_errors():
     with pytest.raises(ValueError, match="out of range"):
         fq.pack_2bit(torch.tensor([[-1, 0, 0, 0]], device=DEV))
     assert fq.pack_2bit(torch.zeros(0, 8, dtype=torch.long, device=DEV)).shape == (0, 2)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n", [1, 300, 2000, 5000, 20000])
+def test_codes_at_a_two_byte_boundary(consts, d, n):
+    """A caller's buffer of codes need only be aligned to two bytes, whichever kernel a call of that size
+    takes; nothing around it is touched."""
+    rot, b4 = consts[f"rotation_{d}_0"], consts[f"boundaries_{d}_4"]
+    x = torch.randn(n, 1, d, generator=torch.Generator().manual_seed(n + d)).to(DEV)
+    want_p, want_n = fq.tq4_compress(x, rot, b4)
+    flat = torch.full((n * d // 2 + 8,), 0xA5, dtype=torch.uint8, device=DEV)
+    packed = flat[2:2 + n * d // 2].view(n, 1, d // 2)
+    norms = torch.empty(n, 1, 1, device=DEV)
+    fq.tq4_compress(x, rot, b4, out=(packed, norms))
+    assert torch.equal(packed, want_p) and torch.equal(norms, want_n)
+    assert bool((flat[:2] == 0xA5).all()) and bool((flat[-6:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("n", [1, 2000, 5000])
+def test_two_stage_codes_at_a_two_byte_boundary(consts, n):
+    rot, s = consts["rotation_128_0"].to(DEV), consts["qjl_128_0"].to(DEV)
+    b3, c3 = consts["boundaries_128_3"].to(DEV), consts["centroids_128_3"].to(DEV)
+    x = torch.randn(n, 128, generator=torch.Generator().manual_seed(n)).to(DEV)
+    want = fq.tq_prod_quantize(x, rot, b3, c3, s)
+    flat = torch.zeros(n * 64 + 8, dtype=torch.uint8, device=DEV)
+    norms, gamma = torch.empty(2, n, device=DEV)
+    bits = torch.empty(n, 16, dtype=torch.uint8, device=DEV)
+    N = fq.kernels.N
+    N.check(N.load().fq_tq_prod_quantize(
+        N.ptr(x), N.dtype_code(x.dtype), N.ptr(rot), N.ptr(b3), b3.numel(), N.ptr(c3), N.ptr(s),
+        flat.data_ptr() + 2, N.ptr(norms), N.ptr(bits), N.ptr(gamma), n, 128, N.stream_ptr(x.device)))
+    assert torch.equal(flat[2:2 + n * 64].view(n, 64), want[0].view(n, 64))
+    assert torch.equal(norms, want[1].flatten()) and torch.equal(bits, want[2].view(n, 16))
+    assert bool((flat[:2] == 0).all()) and bool((flat[-6:] == 0).all())
