@@ -577,7 +577,11 @@ __global__ void __launch_bounds__(kPpThreads, 1) prefill_pair_kernel(PrefillArgs
           const float2 d = f2_unpack(f2_add(s2[2 * c + u], neg2));
           const uint64_t pe = f2_pack(fast_exp2(d.x), fast_exp2(d.y));
           l2 = f2_add(l2, pe);
-          const float2 wf = f2_unpack(f2_mul(pe, u ? vs.y : vs.x));
+          float2 wf = f2_unpack(f2_mul(pe, u ? vs.y : vs.x));
+          if constexpr (decltype(masked)::value) {  // (the norm of a masked token need not be finite)
+            if (d.x == -INFINITY) wf.x = 0.f;
+            if (d.y == -INFINITY) wf.y = 0.f;
+          }
           w[2 * c + u] = pack_half2(wf.x, wf.y);
         }
       }
