@@ -144,15 +144,10 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   // threads r and r + 128 share query row r: the first takes columns 0..31 of a score tile
   // (0..63 of the output), the second the rest; a warp reaches TMEM lanes 32*(warp%4)..+31
   const int row = tid & (kPfM - 1), half = tid >> 7;
-  // heavy (late) query tiles first: the causal work per tile grows with its index
   const bool split_mode = p.n_splits > 1;
-  const int m_tile = split_mode ? 0 : int(gridDim.x) - 1 - int(blockIdx.x);
-  const int split = split_mode ? int(blockIdx.x) : 0;
-  const int hq = blockIdx.y, b = blockIdx.z;
-  const int group = p.hq / p.hkv;
-  const int hkv = hq / group;
-  const int m0 = m_tile * kPfM;
-  const int rows = p.nq - m0 < kPfM ? p.nq - m0 : kPfM;
+  const int split = blockIdx.x;            // slice of the keys
+  const int hkv = blockIdx.y, b = blockIdx.z;
+  const int rows = p.nq;                   // query heads of the KV head: one tile
 
   int kv_end = p.nkv;
   // a slice of the keys: move the bases, the loop below then sees tokens 0 .. kv_end of it
@@ -195,7 +190,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
   }
   // Q tile -> [k-chunk][row][16 B]
   {
-    const __half* qsrc = p.q_rot + ((int64_t(b) * p.hq + hq) * p.nq + m0) * D;
+    const __half* qsrc = p.q_rot + (int64_t(b) * p.hkv + hkv) * p.nq * D;
     for (int i = tid; i < kPfM * int(S::kChunks); i += kPfThreads) {
       const int r = i / int(S::kChunks), kc = i % int(S::kChunks);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -290,7 +285,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
 
   const float k_scale = p.scale_log2 * beta_k, v_scale = 256.f * beta_v;
   float m_run = -INFINITY, l_run = 0.f;
-  const int q_pos = m0 + row;
   bool dead = false;
 
   // ---- prologue: K(0) -> operand, S(0) issued, K(1) and V(0) on their way ------------------
@@ -353,8 +347,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     const float* nk_t = nk_s + (tile & 1) * kPfN;
 
     // ---- online softmax on row `row` ---------------------------------------------------------
-    // A tile that lies wholly below the diagonal of every row of the CTA and is full needs no
-    // masking: the common case gets a loop body without predicates.
+    // a full tile, the common case, gets a loop body without predicates
     const bool unmasked = n_tok == kPfN;
     // pass 1: row maximum of logit*log2e + clamped log2|v| over this thread's half of the tile
     float mx = -INFINITY;
@@ -468,7 +461,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attention_kernel(Prefil
     xch[tid] = l_run;
     __syncthreads();
     const float l_row = l_run + xch[tid ^ kPfM];  // both halves of the row
-    const int64_t row_global = (int64_t(b) * p.hq + hq) * p.nq + q_pos;
+    const int64_t row_global = (int64_t(b) * p.hkv + hkv) * p.nq + row;
     // 2^-kPfPScaleLog2, and 1/l unless the rows of the slices are still to be merged
     const float inv = split_mode ? 1.f / 256.f : (l_row > 0.f ? 1.f / (l_row * 256.f) : 0.f);
     float* dst = split_mode ? p.part + (int64_t(split) * p.total_rows + row_global) * (D + 4)
@@ -552,7 +545,7 @@ static int launch_prefill_t(const PrefillArgs& a, cudaStream_t stream) {
                   cudaGetErrorString(e));
     set_dev = dev;
   }
-  dim3 grid(a.n_splits > 1 ? a.n_splits : (a.nq + kPfM - 1) / kPfM, a.hq, a.batch);
+  dim3 grid(a.n_splits > 1 ? a.n_splits : 1, a.hkv, a.batch);
   kern<<<grid, kPfThreads, S::kBytes, stream>>>(a);
   int rc = check_launch("prefill attention kernel launch");
   if (rc != FQ_OK || a.n_splits <= 1 || a.o_rot == nullptr) return rc;
@@ -730,7 +723,7 @@ static int attention_common(const void* q, fq_dtype dtype, const uint8_t* k_pack
     // One query token: the query heads of a KV group become the rows of one query tile
     // ((B, Hq, 1, D) read as (B, Hkv, group, D)), so the group's keys and values are
     // de-quantised once, and the keys are cut into slices so that the CTAs fill the GPU.
-    a.hq = num_kv_heads; a.nq = group;
+    a.nq = group;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
