@@ -231,3 +231,44 @@ def test_threads_on_one_stream(consts):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_every_call_both_ways(consts, monkeypatch):
+    """The entry points that the extension module takes, and the same through ctypes: the same bits."""
+    w = W.decode_workload(seq_lens=[1, 40, 700], num_q_heads=32, num_kv_heads=8, cfg=64)
+    k, v = (t.to(DEV) for t in W.make_kv(w.total_tokens, 8, 128, 64))
+    rot, bk, bv, ck, cv, qjl = (consts[n].contiguous().to(DEV) for n in (
+        "rotation_128_0", "boundaries_128_3", "boundaries_128_4", "centroids_128_3", "centroids_128_4",
+        "qjl_128_0"))
+    rt = rot.T.contiguous()
+    even, odd = rt[:, 0::2].contiguous(), rt[:, 1::2].contiguous()
+    slots, bt, sl, q = (t.to(DEV) for t in (w.slot_mapping, w.block_table, w.seq_lens, w.q))
+    geo = (8, 128, 16)
+    x = torch.randn(2, 8, 50, 128, device=DEV).to(torch.bfloat16)
+    one = torch.randn(2, 32, 1, 128, device=DEV).to(torch.bfloat16)
+    many = torch.randn(2, 32, 50, 128, device=DEV).to(torch.bfloat16)
+
+    def run():
+        out = list(fq.tq4_compress(k, rot, bk, rotation_T_even=even, rotation_T_odd=odd))
+        cache = torch.zeros(w.num_blocks, 16, 8 * 136, dtype=torch.uint8, device=DEV)
+        plane = torch.zeros(w.num_blocks, 16, 8 * 20, dtype=torch.uint8, device=DEV)
+        fq.tq4_compress_append_qjl(k, v, cache, plane, slots, rot, bk, ck, bv, qjl)
+        out += [cache, plane, fq.split_k_paged_decode_qjl(q, cache, plane, bt, sl, ck, cv, rot, qjl, *geo)]
+        tables = (even, odd, bv, cv, rot)
+        for new in (1, 50):
+            bufs = [torch.zeros(2, 8, 64, n, dtype=t, device=DEV) for n, t in
+                    ((64, torch.uint8), (1, torch.float32)) * 2]
+            K.cache_update(x[:, :, :new].contiguous(), x[:, :, -new:].contiguous(), tables, tables, *bufs, 3)
+            views = [t[:, :, :3 + new] for t in bufs]
+            out += bufs + [fq.fused_tq_attention_kv(one, *views, cv, cv, rot, rot)]
+            read = [torch.zeros(2, 8, 64, 128, dtype=x.dtype, device=DEV) for _ in range(2)]
+            ws = torch.empty(2 * 8 * new * 128 * 4, dtype=torch.uint8, device=DEV)
+            K.cache_update(x[:, :, :new].contiguous(), x[:, :, -new:].contiguous(), tables, tables, *bufs, 3,
+                           *read, 5, ws)
+            out += bufs + read
+        return out + [fq.fused_tq_attention(many, *(t[:, :, 3:53] for t in bufs), cv, cv, rot, is_causal=True)]
+
+    direct = run()
+    monkeypatch.setattr(K, "_host_module", K._ConvertingCalls())
+    for i, (a, b) in enumerate(zip(direct, run())):
+        assert torch.equal(a, b), i
