@@ -623,7 +623,7 @@ def extra_append(ctx):
     return {"us_per_call_two_stage": ms_qjl * 1e3, "us_per_call_one_stage": ms_mse * 1e3,
             "tokens_per_s": 8192 / (ms_qjl * 1e-3), "algorithmic_bytes": alg,
             "hbm_gb_s": alg / (ms_qjl * 1e-3) / 1e9, "frac_of_hbm_peak": alg / (ms_qjl * 1e-3) / 1e9 / peak,
-            "note": "bound by the split-fp16 rotations on mma.sync, not by HBM"}
+            "note": "bound by the element-wise work around the split-fp16 rotations on tcgen05, not by HBM"}
 
 
 def extra_decompress(ctx):
@@ -990,8 +990,9 @@ def run_cache(args):
         "decode_update_us": ms_step * 1e3, "decode_fused_attention_us": ms_attend * 1e3,
         "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s",
                      "frac": gbs / peak, "algorithmic_bytes": alg, "traffic": None,
-                     "note": "two launches of the compress kernel (K, V); the split-fp16 rotation "
-                             "on mma.sync is the binding resource, as for compress-on-append",
+                     "note": "two launches of the compress kernel (K, V); the element-wise work around "
+                             "the split-fp16 rotation is the binding resource, as for "
+                             "compress-on-append",
                      "peak_source": "measured (MEASURED_PEAKS.json)" if peaks else "fallback"},
         "cpu_baseline": cpu,
     }), flush=True)
